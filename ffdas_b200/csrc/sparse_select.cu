@@ -5,15 +5,23 @@
 // (bindings/python/examples/sparse_compounding.py:141-144): per voxel the k
 // events with the largest weight (argpartition over the event axis), then the
 // weights and delays gathered at them (take_along_axis).  This kernel does the
-// same on the device in one pass.  Up to 64 events: a CTA stages the (S, 32)
-// weight and delay blocks of 32 consecutive voxels in shared memory
-// (coalesced rows), each warp sorts a voxel's entries with a 64-element
-// bitonic network over its lanes (two entries per lane, 64-bit keys that
-// carry the order below), and the CTA writes the first k as (k, V) index,
-// weight and delay rows, again coalesced.  More events: one thread per voxel
-// streams the voxel's S weights (consecutive threads read consecutive
-// voxels) and keeps the best KC entries, sorted, in registers with a
-// branch-free compare-and-shift insertion.
+// same on the device in one pass, one thread per voxel: consecutive threads
+// read consecutive voxels, so every row of weights, delays and results is
+// read and written in whole cache lines.  The thread keeps the best KC >= k
+// entries sorted in registers and takes the events KC at a time: it sorts the
+// KC new entries with a merge-exchange network (Batcher, Knuth vol. 3
+// algorithm 5.2.2M), keeps the better of each pair best[i], new[KC-1-i] -- the
+// KC best of both, a bitonic sequence -- and sorts that with log2(KC) levels
+// of half-cleaners.  No lane talks to another and every index is a compile-time
+// constant, so the 2 KC entries stay in registers.
+//
+// Bound by compare-exchange issue (a 64-bit compare and four selects each):
+// for 64 events and k = 32, 494 per voxel (16 of 32 merged pairs keep one side
+// only), against 672 on 64-bit shuffled keys for a warp-wide bitonic sort of
+// 64 entries.  The delays of the tile are copied to shared memory
+// asynchronously while the entries are sorted (column tid of row e lies in
+// bank tid % 32 whatever the lanes' e, so the gather at the end meets no bank
+// conflict).
 //
 // Order: larger weight first, NaN above every number (the host library sorts
 // NaN last in ascending order, so NaN weights are among its k largest), ties
@@ -24,130 +32,131 @@
 
 namespace ffdas {
 
-constexpr int kSelectThreads = 256;
+constexpr int kSelectThreads = 128;
 constexpr int kSelectMaxK = 32;
+// Events whose delays are staged in shared memory (4 bytes x threads each);
+// longer lists gather them from global memory.
+constexpr int kSelectStaged = 96;
 
-// (a, ia) ranks before (b, ib); ib < 0 marks an empty slot, which every entry beats.
-__device__ __forceinline__ bool select_before(float a, int ia, float b, int ib) {
-    if (ib < 0) return true;
-    const bool na = a != a, nb = b != b;
-    if (na != nb) return na;
-    if (!na && a != b) return a > b;
-    return ia < ib;
+// Entry: key orders the weights (larger ranks first), ns is the complement of
+// the event, so that the pair compares as one 64-bit number.
+struct select_entry {
+    uint32_t key, ns;
+};
+
+// The weight's bits mapped to an order-preserving unsigned integer: -0 taken as
+// +0, every NaN above +inf.
+__device__ __forceinline__ uint32_t select_key(float x) {
+    uint32_t u = __float_as_uint(x);
+    if (u == 0x80000000u) u = 0u;
+    return x != x ? 0xffffffffu : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
+}
+
+// a ranks before b: larger key, ties to the lower event.
+__device__ __forceinline__ bool select_before(const select_entry &a, const select_entry &b) {
+    const unsigned long long ka = ((unsigned long long)a.key << 32) | a.ns;
+    const unsigned long long kb = ((unsigned long long)b.key << 32) | b.ns;
+    return ka > kb;
+}
+
+// Compare-exchange: afterwards a ranks before b.
+__device__ __forceinline__ void select_order(select_entry &a, select_entry &b) {
+    const bool ok = select_before(a, b);
+    const select_entry x = a, y = b;
+    a.key = ok ? x.key : y.key;
+    a.ns = ok ? x.ns : y.ns;
+    b.key = ok ? y.key : x.key;
+    b.ns = ok ? y.ns : x.ns;
+}
+
+// Sorts n = 2^m entries, best first: for every p = 1, 2, 4, ... n/2 and
+// k = p, p/2, ... 1 the pairs (j + i, j + i + k) of Batcher's merge exchange.
+template <int KC>
+__device__ __forceinline__ void select_sort(select_entry (&e)[KC]) {
+#pragma unroll
+    for (int p = 1; p < KC; p *= 2) {
+#pragma unroll
+        for (int k = p; k >= 1; k /= 2) {
+#pragma unroll
+            for (int i = 0; i < KC; i++) {
+                // i is the lower index of a pair of this step
+                const int off = i - k % p;
+                if (off >= 0 && (off % (2 * k)) < k && i + k < KC && i / (2 * p) == (i + k) / (2 * p))
+                    select_order(e[i], e[i + k]);
+            }
+        }
+    }
+}
+
+// The KC weights of events s0 .. s0 + KC - 1, and as entries; events past the
+// last rank below every real one (key 0 and a higher event than any).
+template <int KC>
+__device__ __forceinline__ void select_load(const float *__restrict__ w, int s0, int S, int64_t V, float (&x)[KC]) {
+#pragma unroll
+    for (int i = 0; i < KC; i++) x[i] = s0 + i < S ? __ldg(w + (int64_t)(s0 + i) * V) : 0.f;
+}
+template <int KC>
+__device__ __forceinline__ void select_entries(const float (&x)[KC], int s0, int S, select_entry (&e)[KC]) {
+#pragma unroll
+    for (int i = 0; i < KC; i++) {
+        e[i].key = s0 + i < S ? select_key(x[i]) : 0u;
+        e[i].ns = ~(uint32_t)(s0 + i);
+    }
 }
 
 template <int KC>
 __global__ void __launch_bounds__(kSelectThreads) sparse_select_kernel(
-    const float *__restrict__ w, const float *__restrict__ offs, int S, int64_t V, int k,
+    const float *__restrict__ w, const float *__restrict__ offs, int S, int64_t V, int k, bool staged,
     int *__restrict__ idx, float *__restrict__ sw, float *__restrict__ so) {
-    const int64_t v = (int64_t)blockIdx.x * kSelectThreads + threadIdx.x;
+    extern __shared__ float delays[];   // [S][kSelectThreads] when staged; a thread reads its own column only
+    const int tid = threadIdx.x;
+    const int64_t v = (int64_t)blockIdx.x * kSelectThreads + tid;
     if (v >= V) return;
-    float tw[KC];
-    int ti[KC];
-#pragma unroll
-    for (int p = 0; p < KC; p++) {
-        tw[p] = 0.f;
-        ti[p] = -1;
+    if (staged) {
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(delays + tid);
+        for (int s = 0; s < S; s++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(base + (uint32_t)s * (kSelectThreads * 4)),
+                         "l"(offs + (int64_t)s * V + v)
+                         : "memory");
     }
-    for (int s = 0; s < S; s++) {
-        const float x = __ldg(w + (int64_t)s * V + v);
-        // slot p takes slot p-1's entry when the new one ranks before it, the
-        // new entry when it ranks before slot p's (but not slot p-1's), else
-        // keeps its own; slots are updated from the last one down
+    // each group's weights are loaded before the group ahead of it is sorted
+    float x[KC], nx[KC];
+    select_load<KC>(w + v, 0, S, V, x);
+    select_load<KC>(w + v, KC, S, V, nx);
+    select_entry best[KC];
+    select_entries<KC>(x, 0, S, best);
+    select_sort<KC>(best);
+    for (int s0 = KC; s0 < S; s0 += KC) {
+        select_entry e[KC];
+        select_entries<KC>(nx, s0, S, e);
+        if (s0 + KC < S) select_load<KC>(w + v, s0 + KC, S, V, nx);
+        select_sort<KC>(e);
 #pragma unroll
-        for (int p = KC - 1; p > 0; p--) {
-            const bool before_prev = select_before(x, s, tw[p - 1], ti[p - 1]);
-            const bool before_cur = select_before(x, s, tw[p], ti[p]);
-            tw[p] = before_prev ? tw[p - 1] : (before_cur ? x : tw[p]);
-            ti[p] = before_prev ? ti[p - 1] : (before_cur ? s : ti[p]);
+        for (int i = 0; i < KC; i++)
+            if (!select_before(best[i], e[KC - 1 - i])) best[i] = e[KC - 1 - i];
+#pragma unroll
+        for (int d = KC / 2; d >= 1; d /= 2) {
+#pragma unroll
+            for (int i = 0; i < KC; i++)
+                if ((i & d) == 0) select_order(best[i], best[i + d]);
         }
-        const bool first = select_before(x, s, tw[0], ti[0]);
-        tw[0] = first ? x : tw[0];
-        ti[0] = first ? s : ti[0];
     }
+    if (staged) asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
     for (int p = 0; p < KC; p++) {
         if (p < k) {
-            idx[(int64_t)p * V + v] = ti[p];
-            if (sw) sw[(int64_t)p * V + v] = tw[p];
-            if (so) so[(int64_t)p * V + v] = __ldg(offs + (int64_t)ti[p] * V + v);
-        }
-    }
-}
-
-// Sort key of an entry: larger ranks first.  High word: the weight's bits
-// mapped to an order-preserving unsigned integer (-0 taken as +0, every NaN
-// above +inf); low word: ~event, so the lower event ranks first among equal
-// weights.  0 (below every entry) pads a list shorter than 64.
-__device__ __forceinline__ unsigned long long select_key(float x, int s) {
-    uint32_t u = __float_as_uint(x);
-    if (u == 0x80000000u) u = 0u;
-    const uint32_t hi = x != x ? 0xffffffffu : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
-    return ((unsigned long long)hi << 32) | (uint32_t)~(uint32_t)s;
-}
-
-constexpr int kSelectVoxels = 32;           // voxels per CTA (one 128-byte row segment)
-constexpr int kSelectWarps = 8;
-constexpr int kSelectPitch = kSelectVoxels + 1;   // shared rows padded: a warp's column reads meet no conflicts
-
-__global__ void __launch_bounds__(32 * kSelectWarps) sparse_select_warp_kernel(
-    const float *__restrict__ w, const float *__restrict__ offs, int S, int64_t V, int k,
-    int *__restrict__ idx, float *__restrict__ sw, float *__restrict__ so) {
-    __shared__ float tw[64][kSelectPitch], to[64][kSelectPitch];
-    __shared__ int oi[kSelectMaxK][kSelectPitch];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t v0 = (int64_t)blockIdx.x * kSelectVoxels;
-    for (int e = tid; e < S * kSelectVoxels; e += 32 * kSelectWarps) {
-        const int sv = e / kSelectVoxels, c = e % kSelectVoxels;
-        const int64_t v = v0 + c;
-        tw[sv][c] = v < V ? __ldg(w + (int64_t)sv * V + v) : 0.f;
-        if (offs) to[sv][c] = v < V ? __ldg(offs + (int64_t)sv * V + v) : 0.f;
-    }
-    __syncthreads();
-    for (int c = warp; c < kSelectVoxels; c += kSelectWarps) {
-        if (v0 + c >= V) break;   // warp-uniform
-        // entry e = lane + 32 j; ascending bitonic sort of the 64 keys
-        unsigned long long key[2];
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int sv = lane + 32 * j;
-            key[j] = sv < S ? select_key(tw[sv][c], sv) : 0ull;
-        }
-#pragma unroll
-        for (int size = 2; size <= 64; size <<= 1) {
-#pragma unroll
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                if (stride == 32) {   // partner: the lane's other entry (size 64: ascending)
-                    const unsigned long long lo = key[0] < key[1] ? key[0] : key[1];
-                    const unsigned long long hi = key[0] < key[1] ? key[1] : key[0];
-                    key[0] = lo;
-                    key[1] = hi;
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 2; j++) {
-                        const int e = lane + 32 * j;
-                        const unsigned long long other = __shfl_xor_sync(0xffffffffu, key[j], stride);
-                        const bool lower = (e & stride) == 0, up = (e & size) == 0;
-                        const bool keep_small = lower == up;
-                        const bool other_smaller = other < key[j];
-                        key[j] = (keep_small == other_smaller) ? other : key[j];
-                    }
-                }
+            const int64_t o = (int64_t)p * V + v;
+            const uint32_t key = best[p].key, s = ~best[p].ns;
+            idx[o] = (int)s;
+            if (sw) {
+                // the key gives the weight's bits back, except for zeros (either
+                // sign) and NaN payloads, which are read again
+                float x = __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+                if (key == 0x80000000u || key == 0xffffffffu) x = __ldg(w + (int64_t)s * V + v);
+                sw[o] = x;
             }
+            if (so) so[o] = staged ? delays[s * kSelectThreads + tid] : __ldg(offs + (int64_t)s * V + v);
         }
-        // rank p (0 = first) is entry 63 - p: lane 31 - p, j = 1
-        const int p = 31 - lane;
-        if (p < k) oi[p][c] = (int)~(uint32_t)(key[1] & 0xffffffffull);
-    }
-    __syncthreads();
-    for (int e = tid; e < k * kSelectVoxels; e += 32 * kSelectWarps) {
-        const int p = e / kSelectVoxels, c = e % kSelectVoxels;
-        const int64_t v = v0 + c;
-        if (v >= V) continue;
-        const int sv = oi[p][c];
-        idx[(int64_t)p * V + v] = sv;
-        if (sw) sw[(int64_t)p * V + v] = tw[sv][c];
-        if (so) so[(int64_t)p * V + v] = to[sv][c];
     }
 }
 
@@ -156,7 +165,10 @@ static ffdas_error_t launch_select(ffdas_context &h, const float *w, const float
                                    int *idx, float *sw, float *so) {
     const int64_t blocks = (V + kSelectThreads - 1) / kSelectThreads;
     if (blocks > INT32_MAX) return FFDAS_ERROR_DIMS_TOO_LARGE;
-    sparse_select_kernel<KC><<<(unsigned)blocks, kSelectThreads, 0, h.stream>>>(w, offs, S, V, k, idx, sw, so);
+    const bool staged = so && S <= kSelectStaged;
+    const size_t smem = staged ? (size_t)S * kSelectThreads * sizeof(float) : 0;   // at most 48 KB
+    sparse_select_kernel<KC><<<(unsigned)blocks, kSelectThreads, smem, h.stream>>>(w, offs, S, V, k, staged, idx, sw,
+                                                                                   so);
     return ffdas_launch_check(h.stream);
 }
 
@@ -175,15 +187,8 @@ extern "C" ffdas_error_t ffdas_sparse_select(ffdas_handle_t handle, const float 
     if (!weights || !sparse_indices || (sparse_offsets && !offsets)) return FFDAS_ERROR_NULL_POINTER;
     ffdas_context &h = *handle;
     const float *offs = sparse_offsets ? offsets : nullptr;
-    if (n_events <= 64) {
-        const int64_t blocks = (n_voxels + kSelectVoxels - 1) / kSelectVoxels;
-        if (blocks > INT32_MAX) return FFDAS_ERROR_DIMS_TOO_LARGE;
-        sparse_select_warp_kernel<<<(unsigned)blocks, 32 * kSelectWarps, 0, h.stream>>>(
-            weights, offs, n_events, n_voxels, k, sparse_indices, sparse_weights, sparse_offsets);
-        return ffdas_launch_check(h.stream);
-    }
-    if (k <= 1) return launch_select<1>(h, weights, offs, n_events, n_voxels, k, sparse_indices, sparse_weights, sparse_offsets);
-    if (k <= 2) return launch_select<2>(h, weights, offs, n_events, n_voxels, k, sparse_indices, sparse_weights, sparse_offsets);
+    // KC = the smallest power of two from 4 that holds k: the network and the
+    // registers grow with KC, and k entries of KC are written
     if (k <= 4) return launch_select<4>(h, weights, offs, n_events, n_voxels, k, sparse_indices, sparse_weights, sparse_offsets);
     if (k <= 8) return launch_select<8>(h, weights, offs, n_events, n_voxels, k, sparse_indices, sparse_weights, sparse_offsets);
     if (k <= 16) return launch_select<16>(h, weights, offs, n_events, n_voxels, k, sparse_indices, sparse_weights, sparse_offsets);
