@@ -72,6 +72,9 @@ struct ffdas_context {
         int kind = -1;
         const float *scale = nullptr;
         int64_t scale_count = 0;
+        // grid, events and channels of the adjoint's tile plan left in the
+        // buffer's control block (D0 0: none)
+        int D0 = 0, D1 = 0, D2 = 0, events = 0;
     } pair_sig;
     bool last_pairs_reused = false;   // the last ffdas_das_backward read the pair buffer
     int gram_engine = 0;              // ffdas_set_gram_engine: 0 auto, 1 FP32 FMA, 2 tensor cores

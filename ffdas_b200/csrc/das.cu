@@ -16,6 +16,7 @@
 #include "das_problem.h"
 #include "das_direct.h"
 #include "das_gather.cuh"
+#include "das_tile_plan.cuh"
 
 namespace ffdas {
 
@@ -141,7 +142,7 @@ static size_t storage_bytes(int kind) {
 // ---------------------------------------------------------------- ingest ---
 template <typename Tin, int K>
 static ffdas_error_t launch_ingest_t(ffdas_context &h, const das_problem &pb, const void *x,
-                                     int64_t npad, void *P, const float *gain, int gain_bstride) {
+                                     int64_t npad, void *P, const float *gain, int gain_bstride, bool beside_plan) {
     const int64_t rows = (int64_t)pb.B * pb.C * pb.S;
     if (rows == 0) return FFDAS_SUCCESS;
     const int64_t bc = (int64_t)pb.B * pb.C;
@@ -149,9 +150,19 @@ static ffdas_error_t launch_ingest_t(ffdas_context &h, const das_problem &pb, co
     const int64_t per_block = (int64_t)kIngestThreads * kIngestVec;
     dim3 grid((unsigned)((npad + per_block - 1) / per_block), (unsigned)std::min<int64_t>(pb.S, 65535),
               (unsigned)std::min<int64_t>(bc, 65535));
-    ingest_pairs_kernel<Tin, K><<<grid, kIngestThreads, 0, h.stream>>>(
-        static_cast<const Tin *>(x), pb.x_bstride, pb.x_cstride, pb.x_sstride, pb.C, pb.S, pb.N,
-        (int)bc, npad, static_cast<typename pair_traits<K>::storage *>(P), gain, gain_bstride);
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc;
+    std::memset(&lc, 0, sizeof(lc));
+    lc.gridDim = grid;
+    lc.blockDim = dim3(kIngestThreads);
+    lc.stream = h.stream;
+    lc.attrs = &overlap;
+    lc.numAttrs = beside_plan ? 1 : 0;
+    FFDAS_CUDA(cudaLaunchKernelEx(&lc, ingest_pairs_kernel<Tin, K>, static_cast<const Tin *>(x), pb.x_bstride, pb.x_cstride,
+                                  pb.x_sstride, pb.C, pb.S, pb.N, (int)bc, npad,
+                                  static_cast<typename pair_traits<K>::storage *>(P), gain, gain_bstride));
     return ffdas_launch_check(h.stream);
 }
 
@@ -173,12 +184,13 @@ static ffdas_error_t channel_gain(const ffdas_context &h, const das_problem &pb,
     return FFDAS_SUCCESS;
 }
 
+// beside_plan: the launch before is the call's tile plan, which this one overlaps.
 static ffdas_error_t launch_ingest(ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt,
-                                   int kind, const void *x, int64_t npad, void *P) {
+                                   int kind, const void *x, int64_t npad, void *P, bool beside_plan = false) {
     const float *gain = nullptr;
     int gain_bstride = 0;
     FFDAS_TRY(channel_gain(h, pb, &gain, &gain_bstride));
-#define FFDAS_INGEST(Tin, K) launch_ingest_t<Tin, K>(h, pb, x, npad, P, gain, gain_bstride)
+#define FFDAS_INGEST(Tin, K) launch_ingest_t<Tin, K>(h, pb, x, npad, P, gain, gain_bstride, beside_plan)
     switch (xt) {
         case FFDAS_R_32F:
             if (kind == ST_F32) return FFDAS_INGEST(float, ST_F32);
@@ -256,8 +268,8 @@ void *reusable_pairs(const ffdas_context &h, const ffdas_tensor_desc &xd, const 
 }
 
 ffdas_error_t ingest_for_backward(ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt, int kind,
-                                  const void *x, int64_t npad, void *P) {
-    return launch_ingest(h, pb, xt, kind, x, npad, P);
+                                  const void *x, int64_t npad, void *P, bool beside_plan) {
+    return launch_ingest(h, pb, xt, kind, x, npad, P, beside_plan);
 }
 
 // ---------------------------------------------------------------- gather ---
@@ -534,10 +546,36 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     if (h.pair_buf && h.pair_buf_bytes >= pair_bytes + 256) {
         Pbase = h.pair_buf;
     } else {
-        FFDAS_TRY(P.alloc(pair_bytes + (a.sparse ? 256 : 0)));   // das_sparse: a gate word after the pairs
+        FFDAS_TRY(P.alloc(pair_bytes + 256));   // after the pairs: das_sparse's gate word, the tile plan
         Pbase = P.get<void>();
     }
-    FFDAS_TRY(launch_ingest(h, pb, xd.dtype, kind, a.x, npad, Pbase));
+    // without a schedule the staged kernels' tile shape and window width follow
+    // the geometry (das_tile_plan.cuh)
+    const bool staged_ok = staged_supported(pb, kind) && od.dtype == FFDAS_R_32F;
+    schedule s = plan_schedule(h, pb, kind, staged_ok);
+    const int plan_tile = s.variant == 2 && !h.has_config ? s.T0 * s.T1 * s.T2 : 0;
+    const int64_t plan_tiles = plan_tile && pb.C > 0 ? plan_max_tiles(pb, plan_tile) : 0;
+    void *const plan = plan_tiles > 0 && plan_tiles <= INT32_MAX ? static_cast<char *>(Pbase) + pair_bytes + 64 : nullptr;
+    if (plan) {
+        // one item: event chunks of 4 run three CTAs per SM, of 8 two (1024 channels,
+        // 16 events, 128^3 voxels: 7.3 against 8.1 ms; 484 channels, 7 events, 44 x
+        // 59 x 59: 435 against 518 us; a 300 x 256 frame of 16 events, where 8 save
+        // half the passes, 194 against 180)
+        if (pb.B == 1) s.SC = std::min(s.SC, 4);
+        const plan_params own = make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, npad, plan_tile,
+                                          s.BT > 1 ? kPlanBatch : kPlanForward, plan);
+        // pair rows kept for a backward: the adjoint's plan beside the forward's
+        if (Pbase == h.pair_buf && plan_max_tiles(pb, 256) > 0) {
+            const plan_params adjoint = make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, npad, 256, kPlanAdjoint,
+                                                  static_cast<char *>(Pbase) + pair_bytes + 128);
+            FFDAS_TRY(launch_tile_plan(h, own, &adjoint));
+            h.pair_sig.D0 = pb.D0; h.pair_sig.D1 = pb.D1; h.pair_sig.D2 = pb.D2;
+            h.pair_sig.events = pb.n_events;
+        } else {
+            FFDAS_TRY(launch_tile_plan(h, own));
+        }
+    }
+    FFDAS_TRY(launch_ingest(h, pb, xd.dtype, kind, a.x, npad, Pbase, plan != nullptr));
     if (Pbase == h.pair_buf) {
         h.pair_sig.buf = h.pair_buf;
         h.pair_sig.x = a.x;
@@ -548,8 +586,6 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     }
 
     // ---- forward kernel ----
-    const bool staged_ok = staged_supported(pb, kind) && od.dtype == FFDAS_R_32F;
-    const schedule s = plan_schedule(h, pb, kind, staged_ok);
     gather_params gp;
     std::memset(&gp, 0, sizeof(gp));
     gp.P = Pbase;
@@ -615,13 +651,15 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     const bool staged = s.variant == 2;
     if (staged) {
         const int bchunks_st = (pb.B + s.BT - 1) / s.BT;
+        const int64_t tiles = plan ? plan_tiles : (int64_t)gp.n0 * gp.n1 * n2;
+        gp.plan = plan;
         // Small problems (fewer CTAs than the target of min_blocks, default 3,
         // per SM): split each tile's channels over blockIdx.z slices of 32+
         // channels that add into the image, so every SM has work.
         int csplit = 1;
         {
             const int per_sm = (h.has_config && h.config.min_blocks) ? h.config.min_blocks : 3;
-            const int64_t ctas = tiles * bchunks_st;
+            const int64_t ctas = (plan ? plan_min_tiles(pb, plan_tile) : tiles) * bchunks_st;
             const int64_t want = (int64_t)std::max(h.sm_count, 1) * per_sm;
             while (ctas * csplit * 2 <= want && pb.C >= 64 * csplit && csplit < 64) csplit *= 2;
         }
@@ -634,7 +672,8 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         h.last.batch_tile = s.BT;
         h.last.event_chunk = s.SC;
         h.last.grid = tiles * bchunks_st * csplit;
-        h.last.kernels = csplit > 1 ? 3 : 2;   // ingest, (image preparation,) delay-and-sum
+        // (plan,) ingest, (image preparation,) delay-and-sum, (the width not taken)
+        h.last.kernels = (csplit > 1 ? 3 : 2) + (gp.plan ? (s.BT == 1 ? 2 : 1) : 0);
         if (bchunks_st > 65535) return FFDAS_ERROR_DIMS_TOO_LARGE;
         h.mark_start();
         const ffdas_error_t err = launch_staged(h, pb, kind, gp, s.SC, s.WB, s.BT, s.copy,

@@ -21,6 +21,7 @@
 #include "core.h"
 #include "das_problem.h"
 #include "das_pairs.cuh"
+#include "das_tile_plan.cuh"
 
 namespace ffdas {
 
@@ -709,8 +710,35 @@ ffdas_error_t launch_bws_t(ffdas_context &h, const bwd_params &bp, int L, dim3 g
 
 // defined in das.cu
 ffdas_error_t ingest_for_backward(ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt, int kind,
-                                  const void *x, int64_t npad, void *P);
+                                  const void *x, int64_t npad, void *P, bool beside_plan);
 void *reusable_pairs(const ffdas_context &h, const ffdas_tensor_desc &xd, const void *x, int kind);
+
+// One launch for up to four buffers (four memsets cost 2.5 us each on the
+// stream).  Rows of the grid take a buffer each; scalar stores where a buffer
+// is not 16-byte aligned.
+__global__ void __launch_bounds__(256) clear_gradients_kernel(float *a, int64_t na, float *b, int64_t nb, float *c,
+                                                              int64_t nc, float *d, int64_t nd) {
+    float *p = blockIdx.y == 0 ? a : (blockIdx.y == 1 ? b : (blockIdx.y == 2 ? c : d));
+    const int64_t n = blockIdx.y == 0 ? na : (blockIdx.y == 1 ? nb : (blockIdx.y == 2 ? nc : nd));
+    if (!p) return;
+    const int64_t i0 = (int64_t)blockIdx.x * 256 + threadIdx.x, step = (int64_t)gridDim.x * 256;
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        for (int64_t i = i0; i < n / 4; i += step) reinterpret_cast<float4 *>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i0 < (n & 3)) p[(n & ~int64_t(3)) + i0] = 0.f;
+    } else {
+        for (int64_t i = i0; i < n; i += step) p[i] = 0.f;
+    }
+}
+
+ffdas_error_t clear_gradients(ffdas_context &h, float *gw, float *goff, int64_t list_n, float *gdst, int64_t dst_n,
+                              float *gsrc, int64_t src_n) {
+    if (!gw && !goff && !gdst && !gsrc) return FFDAS_SUCCESS;
+    const int64_t most = std::max(std::max((gw || goff) ? list_n : 0, gdst ? dst_n : 0), gsrc ? src_n : 0);
+    const int64_t blocks = std::min<int64_t>((most / 4 + 255) / 256 + 1, 148 * 8);
+    clear_gradients_kernel<<<dim3((unsigned)blocks, 4), 256, 0, h.stream>>>(gw, list_n, goff, list_n, gdst, dst_n, gsrc,
+                                                                          src_n);
+    return ffdas_launch_check(h.stream);
+}
 
 ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tensor_desc &gd,
                            const void *gout, float *gx, float *goff, float *gw, float *gdst, float *gsrc) {
@@ -741,19 +769,37 @@ ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tens
     if (!gout || !a.dstpos || !a.offsets || !a.weights || (pb.C > 0 && !a.srcpos)) return FFDAS_ERROR_NULL_POINTER;
     if (!gx && !goff && !gw && !gdst && !gsrc) return FFDAS_SUCCESS;
 
+    pb.sparse = a.sparse;
     const int64_t npad = pair_row_length(pb.N);
     const int64_t rows = (int64_t)pb.B * pb.C * pb.S;
     const size_t sb = kind == ST_C32 ? 16 : (kind == ST_F32 || kind == ST_C16) ? 8 : 4;
+    const size_t pair_bytes = ((size_t)std::max<int64_t>(rows, 1) * npad * sb + 255) & ~size_t(255);
     // the pair rows of the forward call on this x when it left them in the
-    // handle's pair buffer, else built again
+    // handle's pair buffer (which has 256 bytes after them), else built again
     workspace P(h);
     void *Pbase = reusable_pairs(h, xd, a.x, kind);
     h.last_pairs_reused = Pbase != nullptr;
     if (!Pbase) {
-        FFDAS_TRY(P.alloc((size_t)std::max<int64_t>(rows, 1) * npad * sb));
-        FFDAS_TRY(ingest_for_backward(h, pb, xd.dtype, kind, a.x, npad, P.get<void>()));
+        FFDAS_TRY(P.alloc(pair_bytes + 256));   // after the pairs: the tile plan
         Pbase = P.get<void>();
     }
+    // without a schedule the staged adjoints' tile shape and window width follow
+    // the geometry (das_tile_plan.cuh)
+    pb.sparse = a.sparse;
+    const bool planned_kernel = !h.has_config && !cplx && !a.sparse && !a.srcdir && staged_supported(pb, kind);
+    const int64_t plan_tiles = planned_kernel && pb.C > 0 ? plan_max_tiles(pb, 256) : 0;
+    void *plan = nullptr;
+    if (plan_tiles > 0 && plan_tiles <= INT32_MAX) {
+        // the forward left the adjoint's plan beside its pair rows, if its grid
+        // was this one (a plan for other delays would only be a slower shape)
+        const auto &g = h.pair_sig;
+        const bool kept = h.last_pairs_reused && g.D0 == pb.D0 && g.D1 == pb.D1 && g.D2 == pb.D2 &&
+                          g.events == pb.n_events;
+        plan = static_cast<char *>(Pbase) + pair_bytes + (kept ? 128 : 64);
+        if (!kept)
+            FFDAS_TRY(launch_tile_plan(h, make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, npad, 256, kPlanAdjoint, plan)));
+    }
+    if (!h.last_pairs_reused) FFDAS_TRY(ingest_for_backward(h, pb, xd.dtype, kind, a.x, npad, Pbase, plan != nullptr));
 
     bwd_params bp;
     std::memset(&bp, 0, sizeof(bp));
@@ -779,7 +825,6 @@ ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tens
     bp.gout_bstride = pb.out_bstride;
     bp.gx = gx; bp.goff = goff; bp.gw = gw; bp.gdst = gdst; bp.gsrc = gsrc;
 
-    pb.sparse = a.sparse;
     if (cplx) {   // complex data: the gather-form complex adjoint, one thread per voxel
         const int64_t blocks = (pb.V + kBwdThreads - 1) / kBwdThreads;
         if (blocks > INT32_MAX) return FFDAS_ERROR_DIMS_TOO_LARGE;
@@ -835,8 +880,9 @@ ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tens
             bp.n0 = (pb.D0 + 7) / 8;
             bp.n1 = (pb.D1 + 31) / 32;
         }
-        const int64_t stiles = (int64_t)bp.n0 * bp.n1 * ((pb.D2 + bp.T2 - 1) / bp.T2);
+        int64_t stiles = (int64_t)bp.n0 * bp.n1 * ((pb.D2 + bp.T2 - 1) / bp.T2);
         if (stiles > INT32_MAX) return FFDAS_ERROR_DIMS_TOO_LARGE;
+        if (plan) stiles = plan_tiles;
         // batch tiles: up to 4 items per CTA share each window's delays
         const int WB = (h.has_config && h.config.window > 32) ? 64 : 32;
         const int copy = h.has_config ? h.config.copy_engine : 0;
@@ -852,7 +898,7 @@ ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tens
         int csplit = 1;
         {
             const int per_sm = (h.has_config && h.config.min_blocks) ? h.config.min_blocks : 2;
-            const int64_t ctas = stiles * bchunks_st;
+            const int64_t ctas = (plan ? plan_min_tiles(pb, 256) : stiles) * bchunks_st;
             const int64_t want = (int64_t)std::max(h.sm_count, 1) * per_sm;
             while (ctas * csplit * 2 <= want && pb.C >= 64 * csplit && csplit < 64) csplit *= 2;
         }
@@ -862,13 +908,10 @@ ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tens
             csplit = (pb.C + cchunk - 1) / cchunk;
             if (csplit < 2) cchunk = 0;
         }
-        const size_t ve0 = (size_t)pb.n_events * pb.V * sizeof(float);
-        if (pb.B > 1 || csplit > 1) {  // several CTAs add into the voxel-side gradients
-            if (gw) FFDAS_CUDA(cudaMemsetAsync(gw, 0, ve0, h.stream));
-            if (goff) FFDAS_CUDA(cudaMemsetAsync(goff, 0, ve0, h.stream));
-            if (gdst) FFDAS_CUDA(cudaMemsetAsync(gdst, 0, (size_t)pb.V * 3 * sizeof(float), h.stream));
-        }
-        if (gsrc) FFDAS_CUDA(cudaMemsetAsync(gsrc, 0, (size_t)pb.C * 3 * sizeof(float), h.stream));
+        // several CTAs add into the voxel-side gradients, all into the channels'
+        const bool shared_v = pb.B > 1 || csplit > 1;
+        FFDAS_TRY(clear_gradients(h, shared_v ? gw : nullptr, shared_v ? goff : nullptr, (int64_t)pb.n_events * pb.V,
+                                  shared_v ? gdst : nullptr, pb.V * 3, gsrc, (int64_t)pb.C * 3));
         gather_params gp;
         std::memset(&gp, 0, sizeof(gp));
         gp.P = Pbase;
@@ -879,12 +922,14 @@ ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tens
         gp.srcpos = a.srcpos; gp.dstpos = a.dstpos; gp.offsets = a.offsets; gp.weights = a.weights;
         gp.beta_zero = 1;
         gp.cchunk = cchunk;
+        gp.plan = plan;
         const staged_grads gr{static_cast<const float *>(gout), pb.out_bstride, gx, goff, gw, gdst, gsrc};
         h.last = ffdas_kernel_info_t{};
         h.last.variant = 4;
         h.last.tile_x = bp.T0; h.last.tile_y = bp.T1; h.last.tile_z = bp.T2;
         h.last.batch_tile = BT; h.last.event_chunk = SC; h.last.storage = kind;
-        h.last.kernels = h.last_pairs_reused ? 1 : 2;   // (ingest,) adjoint
+        // (ingest,) adjoint; the plan and the width not taken are not counted
+        h.last.kernels = h.last_pairs_reused ? 1 : 2;
         h.last.grid = stiles * bchunks_st * csplit;
         if (bchunks_st > 65535) return FFDAS_ERROR_DIMS_TOO_LARGE;
         h.mark_start();

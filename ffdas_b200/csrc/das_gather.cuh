@@ -42,6 +42,7 @@ struct gather_params {
     double beta_re, beta_im;
     int beta_zero;
     int cchunk;               // staged forward: channels per blockIdx.z slice (0: no split)
+    void *plan;               // staged kernels: device word block of the planned tile shape, or null
     const int *run_if;        // when set, the kernel runs only if *run_if != 0 (das_sparse fallback)
 };
 

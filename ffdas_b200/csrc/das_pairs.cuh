@@ -243,6 +243,8 @@ __global__ void __launch_bounds__(kIngestThreads) ingest_pairs_kernel(
             *reinterpret_cast<pair_quad<st> *>(P + ((int64_t)bc * S + s) * Npad + k0) = q;
         }
     }
+    // launched beside the tile plan: complete only after it (no-op else)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 }  // namespace ffdas

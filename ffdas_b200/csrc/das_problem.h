@@ -77,8 +77,26 @@ bool staged_batch_supported();
 // channel slices add into it.
 ffdas_error_t launch_scale_image(ffdas_context &h, const das_problem &pb, float *out, float beta, int beta_zero);
 // BT > 1: batch tiles of BT items per CTA (256-voxel tiles, SC * BT <= 32).
+// With gp.plan set the tile shape and the window width come from the plan
+// made there; grid.x is then plan_max_tiles().
 ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp, int SC,
                             int WB, int BT, int copy, dim3 grid);
+
+// Most tiles of any candidate shape of `tile_voxels` voxels; 0 when the grid
+// admits none (then no plan).
+int64_t plan_max_tiles(const das_problem &pb, int tile_voxels);
+// Fewest tiles of any candidate: the plan avoids padding, so this is near the
+// count it ends with, and the one to split channels by (283 x 142 pixels: 512 x 1
+// tiles would be 283, 32 x 16 ones 81; slices for 283 left half the SMs idle).
+int64_t plan_min_tiles(const das_problem &pb, int tile_voxels);
+// what the shape is chosen for: one item, batch tiles, the adjoints, the products
+enum : int { kPlanForward = 0, kPlanAdjoint = 1, kPlanMma = 2, kPlanBatch = 3 };
+// The inputs of a plan written to `plan` (device memory), and the launch that
+// makes one, or two.
+struct plan_params;
+plan_params make_plan(const das_problem &pb, int kind, const float *srcpos, const float *dstpos, const float *offsets,
+                      int64_t npad, int tile_voxels, int mode, void *plan);
+ffdas_error_t launch_tile_plan(ffdas_context &h, const plan_params &own, const plan_params *adjoint = nullptr);
 
 // Gradient outputs of the staged adjoint kernel (null = not computed).
 struct staged_grads {
@@ -86,6 +104,10 @@ struct staged_grads {
     int64_t gout_bstride;
     float *gx, *goff, *gw, *gdst, *gsrc;
 };
+// Zeroes the given gradient outputs (null: none) in one launch: gw and goff of
+// list_n floats, gdst of dst_n, gsrc of src_n.
+ffdas_error_t clear_gradients(ffdas_context &h, float *gw, float *goff, int64_t list_n, float *gdst, int64_t dst_n,
+                              float *gsrc, int64_t src_n);
 // Complex (IQ) data on the staged kernel: 256-voxel tiles, 32-pair windows,
 // TMA copies, event chunk 4 or 8.
 ffdas_error_t launch_staged_cplx(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp,

@@ -16,6 +16,8 @@
 #include "core.h"
 #include "das_problem.h"
 #include "das_staged.cuh"
+#include "das_tile_plan.cuh"
+#include "das_staged_host.cuh"
 #include "das_sparse_items.cuh"
 
 namespace ffdas {
@@ -60,7 +62,7 @@ static int staged_pair_bytes(int kind) {
 // 2-D map over the pair rows (one row per item, channel, event); a 16-byte
 // (complex f32) pair is two 8-byte elements, so its x coordinates and box
 // width count elements, not pairs.
-static ffdas_error_t pair_row_map(CUtensorMap &map, const void *P, int64_t npad, int64_t rows, int kind, int WB) {
+ffdas_error_t pair_row_map(CUtensorMap &map, const void *P, int64_t npad, int64_t rows, int kind, int WB) {
     auto encode = tensor_map_encoder();
     if (!encode) return FFDAS_ERROR_CUDA_DRIVER;
     const int pair_bytes = staged_pair_bytes(kind);
@@ -77,17 +79,18 @@ static ffdas_error_t pair_row_map(CUtensorMap &map, const void *P, int64_t npad,
 }
 
 // 3-D map over the same rows for batch tiles: dims {npad, C*S, B}, box
-// {WB, 1, BT}; batch items past B read as zeros.
-static ffdas_error_t pair_batch_map(CUtensorMap &map, const void *P, int64_t npad, int64_t cs, int64_t B, int kind,
+// {WB, 1, BT}; batch items past B read as zeros.  16-byte pairs as above.
+ffdas_error_t pair_batch_map(CUtensorMap &map, const void *P, int64_t npad, int64_t cs, int64_t B, int kind,
                                     int WB, int BT) {
     auto encode = tensor_map_encoder();
     if (!encode) return FFDAS_ERROR_CUDA_DRIVER;
-    const int pair_bytes = (kind == ST_F32) ? 8 : 4;
-    const cuuint64_t dims[3] = {(cuuint64_t)npad, (cuuint64_t)cs, (cuuint64_t)B};
+    const int pair_bytes = staged_pair_bytes(kind);
+    const int units = pair_bytes == 16 ? 2 : 1;
+    const cuuint64_t dims[3] = {(cuuint64_t)(npad * units), (cuuint64_t)cs, (cuuint64_t)B};
     const cuuint64_t strides[2] = {(cuuint64_t)npad * pair_bytes, (cuuint64_t)(cs * npad * pair_bytes)};
-    const cuuint32_t box[3] = {(cuuint32_t)WB, 1u, (cuuint32_t)BT};
+    const cuuint32_t box[3] = {(cuuint32_t)(WB * units), 1u, (cuuint32_t)BT};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
-    const CUresult r = encode(&map, pair_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32,
+    const CUresult r = encode(&map, pair_bytes >= 8 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32,
                               3, const_cast<void *>(P), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -95,29 +98,6 @@ static ffdas_error_t pair_batch_map(CUtensorMap &map, const void *P, int64_t npa
 }
 
 bool staged_batch_supported() { return tensor_map_encoder() != nullptr; }
-
-template <typename Kernel>
-static ffdas_error_t prepare_kernel(Kernel kernel, size_t smem) {
-    FFDAS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // all of the unified L1/shared array as shared memory: several CTAs per SM
-    FFDAS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    (int)cudaSharedmemCarveoutMaxShared));
-    return FFDAS_SUCCESS;
-}
-
-// Kernel attributes (dynamic shared memory above 48 KB, carveout) belong to a
-// device: set them once for every device the process launches the kernel on.
-template <auto Kernel>
-static ffdas_error_t prepare_once(size_t smem) {
-    static std::atomic<unsigned long long> done{0ull};
-    int dev = 0;
-    FFDAS_CUDA(cudaGetDevice(&dev));
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done.load(std::memory_order_acquire) & bit) return FFDAS_SUCCESS;
-    FFDAS_TRY(prepare_kernel(Kernel, smem));
-    done.fetch_or(bit, std::memory_order_release);
-    return FFDAS_SUCCESS;
-}
 
 template <int K, int SC, int WB>
 static ffdas_error_t launch_fwd_t(ffdas_context &h, const staged_params &sp, const CUtensorMap &map, dim3 grid) {
@@ -202,7 +182,7 @@ static ffdas_error_t launch_bwd_sc(ffdas_context &h, const staged_params &sp, co
     return SC == 1 ? launch_bwd_t<K, 1, WB>(h, sp, map, grid) : launch_bwd_t<K, 4, WB>(h, sp, map, grid);
 }
 
-static staged_params base_params(ffdas_context &h, const das_problem &pb, const gather_params &gp) {
+staged_params base_params(ffdas_context &h, const das_problem &pb, const gather_params &gp) {
     staged_params sp;
     std::memset(&sp, 0, sizeof(sp));
     sp.P = gp.P;
@@ -219,6 +199,7 @@ static staged_params base_params(ffdas_context &h, const das_problem &pb, const 
     sp.units = h.timing ? h.unit_count : nullptr;
     sp.debug_drop_stage = ffdas_take_debug_drop_stage();
     sp.cchunk = gp.cchunk;
+    sp.plan = static_cast<const tile_plan *>(gp.plan);
     return sp;
 }
 
@@ -227,6 +208,62 @@ ffdas_error_t launch_scale_image(ffdas_context &h, const das_problem &pb, float 
     scale_image_kernel<<<sg, 256, 0, h.stream>>>(out, pb.out_bstride, pb.V, pb.B, beta, beta_zero, nullptr);
     return ffdas_launch_check(h.stream);
 }
+
+// Candidate tiles of `tile_voxels` voxels (a power of two) over the two
+// innermost grid axes, widest first, none more than twice as long as its axis.
+static int plan_candidates(const das_problem &pb, int tile_voxels, int *T0, int *T1) {
+    int n = 0;
+    for (int t0 = tile_voxels; t0 >= 4 && n < kPlanShapes; t0 >>= 1) {
+        const int t1 = tile_voxels / t0;
+        if ((t0 >= 2 * pb.D0 && t0 > 4) || (t1 >= 2 * pb.D1 && t1 > 1)) continue;
+        T0[n] = t0;
+        T1[n++] = t1;
+    }
+    return n;
+}
+
+int64_t plan_max_tiles(const das_problem &pb, int tile_voxels) {
+    int T0[kPlanShapes], T1[kPlanShapes];
+    int64_t most = 0;
+    const int n = plan_candidates(pb, tile_voxels, T0, T1);
+    for (int i = 0; i < n; i++)
+        most = std::max(most, (int64_t)((pb.D0 + T0[i] - 1) / T0[i]) * ((pb.D1 + T1[i] - 1) / T1[i]) * pb.D2);
+    return most;
+}
+
+int64_t plan_min_tiles(const das_problem &pb, int tile_voxels) {
+    int T0[kPlanShapes], T1[kPlanShapes];
+    int64_t least = INT64_MAX;
+    const int n = plan_candidates(pb, tile_voxels, T0, T1);
+    for (int i = 0; i < n; i++)
+        least = std::min(least, (int64_t)((pb.D0 + T0[i] - 1) / T0[i]) * ((pb.D1 + T1[i] - 1) / T1[i]) * pb.D2);
+    return n ? least : 0;
+}
+
+plan_params make_plan(const das_problem &pb, int kind, const float *srcpos, const float *dstpos, const float *offsets,
+                      int64_t npad, int tile_voxels, int mode, void *plan) {
+    plan_params q;
+    std::memset(&q, 0, sizeof(q));
+    q.srcpos = srcpos; q.dstpos = dstpos; q.offsets = offsets;
+    q.C = pb.C; q.n_events = pb.n_events; q.V = pb.V; q.npad = npad;
+    // pairs per 16 bytes; complex windows hold plain samples, where a tap needs
+    // its next one too
+    q.align = kind == ST_C32 ? 3 : kind == ST_C16 ? 5 : std::max(1, 16 / staged_pair_bytes(kind));
+    q.D0 = pb.D0; q.D1 = pb.D1; q.D2 = pb.D2;
+    q.shapes = plan_candidates(pb, tile_voxels, q.T0, q.T1);
+    q.mode = mode;
+    q.plan = static_cast<tile_plan *>(plan);
+    return q;
+}
+
+ffdas_error_t launch_tile_plan(ffdas_context &h, const plan_params &own, const plan_params *adjoint) {
+    if (own.shapes == 0 || own.C < 1 || own.n_events < 1 || (adjoint && adjoint->shapes == 0)) return FFDAS_ERROR_INTERNAL;
+    tile_plan_kernel<<<adjoint ? 2 : 1, 256, 0, h.stream>>>(own, adjoint ? *adjoint : own);
+    return ffdas_launch_check(h.stream);
+}
+
+static ffdas_error_t launch_staged_width(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp,
+                                         int SC, int WB, int BT, int copy, dim3 grid);
 
 ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp, int SC,
                             int WB, int BT, int copy, dim3 grid) {
@@ -237,6 +274,13 @@ ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, c
                                                      (float)gp.beta_re, gp.beta_zero, nullptr);
         FFDAS_TRY(ffdas_launch_check(h.stream));
     }
+    if (!gp.plan || BT > 1) return launch_staged_width(h, pb, kind, gp, SC, BT > 1 && gp.plan ? 64 : WB, BT, copy, grid);
+    FFDAS_TRY(launch_staged_width(h, pb, kind, gp, SC, 32, BT, copy, grid));
+    return launch_staged_width(h, pb, kind, gp, SC, 64, BT, copy, grid);
+}
+
+static ffdas_error_t launch_staged_width(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp,
+                                         int SC, int WB, int BT, int copy, dim3 grid) {
     if (BT > 1) copy = 1;   // batch tiles stage their windows with 3-D TMA boxes
     copy = resolve_copy(copy);
     if (BT > 1 && copy != 1) return FFDAS_ERROR_CUDA_DRIVER;
@@ -250,6 +294,14 @@ ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, c
     sp.copy_async = copy == 2;
     h.last.copy_engine = copy;
     if (BT > 1) {
+        // A plan has fewer tiles than the launch, which is sized for any: with the
+        // batch chunks innermost the CTAs left over come last (between the chunks
+        // they cost a batch of 32 items 7 %: 646 against 605 us on 155 tiles of a
+        // launch for 248).
+        if (gp.plan && grid.y > 1 && grid.x <= 65535) {
+            std::swap(grid.x, grid.y);
+            sp.tile_y = 1;
+        }
         switch (kind) {
             case ST_F32:
                 return WB == 64 ? launch_fwd_batch<ST_F32, 64>(h, sp, map, SC, BT, grid)
@@ -466,8 +518,20 @@ ffdas_error_t launch_sparse_items(ffdas_context &h, const das_problem &pb, int k
     }
 }
 
+static ffdas_error_t launch_staged_bwd_width(ffdas_context &h, const das_problem &pb, int kind,
+                                             const gather_params &gp, const staged_grads &gr, int SC, int WB, int BT,
+                                             int copy, dim3 grid);
+
 ffdas_error_t launch_staged_bwd(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp,
                                 const staged_grads &gr, int SC, int WB, int BT, int copy, dim3 grid) {
+    if (!gp.plan) return launch_staged_bwd_width(h, pb, kind, gp, gr, SC, WB, BT, copy, grid);
+    FFDAS_TRY(launch_staged_bwd_width(h, pb, kind, gp, gr, SC, 32, BT, copy, grid));
+    return launch_staged_bwd_width(h, pb, kind, gp, gr, SC, 64, BT, copy, grid);
+}
+
+static ffdas_error_t launch_staged_bwd_width(ffdas_context &h, const das_problem &pb, int kind,
+                                             const gather_params &gp, const staged_grads &gr, int SC, int WB, int BT,
+                                             int copy, dim3 grid) {
     if (BT > 1) copy = 1;   // batch tiles stage their windows with 3-D TMA boxes
     copy = resolve_copy(copy);
     if (BT > 1 && copy != 1) return FFDAS_ERROR_CUDA_DRIVER;

@@ -45,7 +45,17 @@ constexpr uint32_t kOvf = 0xFFFFFFFFu;     // meta value: window wider than a sl
 constexpr long long kWaitCycles = 4000000000LL;  // ~2 s at 2 GHz
 constexpr int kStatusTimeout = 1;
 
+// Tile shape and window width of a call whose schedule the planner leaves to
+// the geometry (tile_plan_kernel): written on the device before the staged
+// kernels run.  One instance per window width is launched; the other exits.
+struct __align__(16) tile_plan {
+    int T0, T1, n0, n1;   // T2 = 1
+    int wb;
+};
+
 struct staged_params {
+    const tile_plan *plan;   // null: the shape below, whatever the kernel's window width
+    int tile_y;              // batch tiles: the tile is blockIdx.y, the batch chunk blockIdx.x (0: the other way round)
     const void *P;
     int64_t npad;
     int C, S, N, n_events, B;
@@ -74,6 +84,23 @@ struct staged_params {
     int64_t gout_bstride;
     float *gx, *goff, *gw, *gdst, *gsrc;
 };
+
+// The tile shape of a launch: the planned one, or the launch's own.  (Beside the
+// parameters, not in a modified copy of them, which held more registers: batch
+// tiles 627 against 605 us.  das_staged2_kernel is the other way round, see there.)
+struct tile_shape {
+    int T0, T1, T2, n0, n1;
+};
+// False: this instance, or this CTA, has no tile (uniform over the CTA, before
+// any barrier or copy).
+template <int WB, bool TILE_Y = false>
+__device__ __forceinline__ bool take_plan(const staged_params &p, tile_shape &t) {
+    t = {p.T0, p.T1, p.T2, p.n0, p.n1};
+    if (!p.plan) return true;
+    const int4 q = *reinterpret_cast<const int4 *>(p.plan);
+    t = {q.x, q.y, 1, q.z, q.w};
+    return p.plan->wb == WB && (int64_t)(TILE_Y && p.tile_y ? blockIdx.y : blockIdx.x) < (int64_t)q.z * q.w * p.D2;
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -115,6 +142,13 @@ __device__ __forceinline__ void tma_load_box3(uint32_t dst, const CUtensorMap *m
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+// Box {WB samples, 1 event, G channels, BT items} of a 4-D map over sample rows.
+__device__ __forceinline__ void tma_load_box4(uint32_t dst, const CUtensorMap *map, int k, int s, int c, int b,
+                                              uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(k), "r"(s), "r"(c), "r"(b), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void consumer_sync() {
     asm volatile("bar.sync 1, %0;" ::"r"(kStConsumers) : "memory");
@@ -339,9 +373,10 @@ struct staged_smem {
     int *flags;            // [4]: -, voxel and channel positions finite, pass flags (by pass parity)
     unsigned char *extra;  // adjoint scratch
 
-    __device__ explicit staged_smem(unsigned char *raw) {
+    // ring_bytes: a ring of another layout (das_iq.cuh)
+    __device__ explicit staged_smem(unsigned char *raw, size_t ring_bytes = SG::ring_bytes) {
         ring = raw;
-        zslot = ring + SG::ring_bytes;
+        zslot = ring + ring_bytes;
         meta = reinterpret_cast<uint32_t *>(zslot + SG::bytes);
         ovf = reinterpret_cast<int *>(meta + kStages * kStWin);
         full = reinterpret_cast<uint64_t *>(ovf + kStages);
@@ -391,8 +426,9 @@ struct staged_ctx {
 // (the adjoint's scatter then meets few same-address atomics).
 // With vt == 2 the tile holds 512 voxels and each consumer thread also owns
 // the voxel 256 places further in the tile's linear order.
-template <int K, int WB>
-__device__ __forceinline__ staged_ctx staged_setup(const staged_params &p, staged_smem<K, WB> &sm,
+// PAD: the ring holds padded slots, whose zero pairs are written here.
+template <int K, int WB, bool PAD = true, bool TILE_Y = false>
+__device__ __forceinline__ staged_ctx staged_setup(const staged_params &p, const tile_shape &t, staged_smem<K, WB> &sm,
                                                    bool spread = false, int vt = 1) {
     using SG = slot_geom<WB, K>;
     staged_ctx cx;
@@ -400,7 +436,7 @@ __device__ __forceinline__ staged_ctx staged_setup(const staged_params &p, stage
     cx.warp = cx.tid >> 5;
     cx.lane = cx.tid & 31;
     cx.producer = (cx.warp == kStWarps);
-    cx.b = blockIdx.y;
+    cx.b = TILE_Y && p.tile_y ? blockIdx.x : blockIdx.y;
     cx.active = false;
     cx.v = 0;
     cx.vx = cx.vy = cx.vz = 0.f;
@@ -408,19 +444,19 @@ __device__ __forceinline__ staged_ctx staged_setup(const staged_params &p, stage
     cx.active2 = false;
     cx.v2 = 0;
     cx.vx2 = cx.vy2 = cx.vz2 = 0.f;
-    const int tile = blockIdx.x;
-    const int t0 = tile % p.n0, t1 = (tile / p.n0) % p.n1, t2 = tile / (p.n0 * p.n1);
+    const int tile = TILE_Y && p.tile_y ? blockIdx.y : blockIdx.x;
+    const int t0 = tile % t.n0, t1 = (tile / t.n0) % t.n1, t2 = tile / (t.n0 * t.n1);
     if (!cx.producer) {
         const int lt = spread ? (cx.lane * kStWarps + cx.warp) : cx.tid;
-        const int i0 = lt % p.T0, i1 = (lt / p.T0) % p.T1, i2 = lt / (p.T0 * p.T1);
-        const int g0 = t0 * p.T0 + i0, g1 = t1 * p.T1 + i1, g2 = t2 * p.T2 + i2;
+        const int i0 = lt % t.T0, i1 = (lt / t.T0) % t.T1, i2 = lt / (t.T0 * t.T1);
+        const int g0 = t0 * t.T0 + i0, g1 = t1 * t.T1 + i1, g2 = t2 * t.T2 + i2;
         cx.par = (i0 + i1 + i2) & 1;
         cx.active = (g0 < p.D0 && g1 < p.D1 && g2 < p.D2);
         // 512-voxel tiles: a voxel past the grid stands in for the tile's
         // first voxel (always inside the grid) -- same position and delays,
         // weight 0, no output -- so every thread's taps stay inside the
         // windows the producer bounds from the tile's voxels
-        const int64_t v_first = ((int64_t)(t2 * p.T2) * p.D1 + t1 * p.T1) * p.D0 + t0 * p.T0;
+        const int64_t v_first = ((int64_t)(t2 * t.T2) * p.D1 + t1 * t.T1) * p.D0 + t0 * t.T0;
         if (cx.active || vt == 2) {
             cx.v = cx.active ? ((int64_t)g2 * p.D1 + g1) * p.D0 + g0 : v_first;
             cx.vx = __ldg(p.dstpos + 3 * cx.v);
@@ -429,8 +465,8 @@ __device__ __forceinline__ staged_ctx staged_setup(const staged_params &p, stage
         }
         if (vt == 2) {
             const int lt2 = lt + kStConsumers;
-            const int j0 = lt2 % p.T0, j1 = (lt2 / p.T0) % p.T1, j2 = lt2 / (p.T0 * p.T1);
-            const int h0 = t0 * p.T0 + j0, h1 = t1 * p.T1 + j1, h2 = t2 * p.T2 + j2;
+            const int j0 = lt2 % t.T0, j1 = (lt2 / t.T0) % t.T1, j2 = lt2 / (t.T0 * t.T1);
+            const int h0 = t0 * t.T0 + j0, h1 = t1 * t.T1 + j1, h2 = t2 * t.T2 + j2;
             cx.active2 = (h0 < p.D0 && h1 < p.D1 && h2 < p.D2);
             cx.v2 = cx.active2 ? ((int64_t)h2 * p.D1 + h1) * p.D0 + h0 : v_first;
             cx.vx2 = __ldg(p.dstpos + 3 * cx.v2);
@@ -448,7 +484,7 @@ __device__ __forceinline__ staged_ctx staged_setup(const staged_params &p, stage
         *sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    {
+    if constexpr (PAD) {
         constexpr int zwords = (SG::bytes - SG::data_bytes) / 4;
         for (int i = cx.tid; i < kStages * kStWin * zwords; i += kStThreads) {
             const int slot = i / zwords, word = i - slot * zwords;
@@ -1147,7 +1183,7 @@ __global__ void __launch_bounds__(kStThreads) das_staged_kernel(const staged_par
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     staged_smem<K, WB> sm(smem_raw);
-    const staged_ctx cx = staged_setup<K, WB>(p, sm);
+    const staged_ctx cx = staged_setup<K, WB>(p, tile_shape{p.T0, p.T1, p.T2, p.n0, p.n1}, sm);
 
     const st *__restrict__ Pg = static_cast<const st *>(p.P);
     const uint32_t kmax_pair = (uint32_t)(p.npad - 1);
@@ -1293,8 +1329,17 @@ __global__ void __launch_bounds__(kStThreads) das_staged_kernel(const staged_par
 // index onto the slot's zero pair as before.  Every variant reads the same
 // pair for every tap, so the image is bit-identical across them.
 template <int K, int SC, int WB>
-__global__ void __launch_bounds__(kStThreads, SC >= 8 ? 2 : 3) das_staged2_kernel(const staged_params p,
+__global__ void __launch_bounds__(kStThreads, SC >= 8 ? 2 : 3) das_staged2_kernel(const staged_params params,
                                                                   const __grid_constant__ CUtensorMap tmap) {
+    // (a modified copy of the parameters: four events of FP32 pairs then spill
+    // nothing, 16 bytes with the shape beside them -- 223 against 255 us where a
+    // third of the windows overflow)
+    staged_params p = params;
+    {
+        tile_shape shape;
+        if (!take_plan<WB>(p, shape)) return;
+        p.T0 = shape.T0; p.T1 = shape.T1; p.T2 = shape.T2; p.n0 = shape.n0; p.n1 = shape.n1;
+    }
     using st = typename pair_traits<K>::storage;
     using SG = slot_geom<WB, K>;
     constexpr int CC = kStWin / SC;  // channels per stage
@@ -1306,7 +1351,7 @@ __global__ void __launch_bounds__(kStThreads, SC >= 8 ? 2 : 3) das_staged2_kerne
     if (p.gate && *(volatile const int *)p.gate) return;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     staged_smem<K, WB> sm(smem_raw);
-    const staged_ctx cx = staged_setup<K, WB>(p, sm, false, 2);
+    const staged_ctx cx = staged_setup<K, WB>(p, tile_shape{p.T0, p.T1, p.T2, p.n0, p.n1}, sm, false, 2);
     const int n_active = staged_tile_bounds<K, WB>(p, sm, cx);
     const int cbeg = chan_begin(p), cend = chan_end(p);   // this CTA's channel slice
 
@@ -1376,13 +1421,16 @@ __global__ void __launch_bounds__(kStThreads, SC >= 8 ? 2 : 3) das_staged2_kerne
                                 acc2 = __ffma2_rn(w2[j], make_float2(ta, tb), acc2);
                             }
                         }
-                    } else if (!any_ovf && !p.srcdir) {
-                        // No per-channel branch; tap indices are clamped onto the
+                    } else if (!any_ovf) {
+                        // No per-voxel branch; tap indices are clamped onto the
                         // slot's zero pair.  The channel table's (x, x, y, y),
                         // (z, z, 0, 0) rows feed the packed geometry directly:
                         // d = c - v, the exact negative of v - c, so rsq is the
                         // same as receive_geometry's.  Channels past C carry a
-                        // zero window: their taps read the zero pair.
+                        // zero window: their taps read the zero pair.  With element
+                        // directivity a voxel outside the channel's cone gets the
+                        // delay 1e30, whose index clamps onto the zero pair too.
+                        auto channels = [&](auto with_dir) {
 #pragma unroll
                         for (int cl = 0; cl < CC; cl++) {
                             const float4 qa = lds_f4(pair_u32 + (stage * kStWin + cl) * 32);
@@ -1393,8 +1441,18 @@ __global__ void __launch_bounds__(kStThreads, SC >= 8 ? 2 : 3) das_staged2_kerne
                             float2 r2 = __fmul2_rn(dx, dx);
                             r2 = __ffma2_rn(dy, dy, r2);
                             r2 = __ffma2_rn(dz, dz, r2);
-                            const float2 rsq2 = make_float2(fmaxf(r2.x, 1e-7f), fmaxf(r2.y, 1e-7f));
-                            const float2 rinv2 = make_float2(rsqrtf(rsq2.x), rsqrtf(rsq2.y));
+                            float2 rsq2 = make_float2(fmaxf(r2.x, 1e-7f), fmaxf(r2.y, 1e-7f));
+                            float2 rinv2 = make_float2(rsqrtf(rsq2.x), rsqrtf(rsq2.y));
+                            if constexpr (decltype(with_dir)::value) {
+                                // the cosine of apply_directivity, negated with d
+                                const float4 dir = sm.chan_dir[stage * kStWin + cl];
+                                float2 pr2 = __fmul2_rn(dx, make_float2(dir.x, dir.x));
+                                pr2 = __ffma2_rn(dy, make_float2(dir.y, dir.y), pr2);
+                                pr2 = __ffma2_rn(dz, make_float2(dir.z, dir.z), pr2);
+                                const bool ina = -(pr2.x * rinv2.x) > dir.w, inb = -(pr2.y * rinv2.y) > dir.w;
+                                rsq2 = make_float2(ina ? rsq2.x : 1e30f, inb ? rsq2.y : 1e30f);
+                                rinv2 = make_float2(ina ? rinv2.x : 1.f, inb ? rinv2.y : 1.f);
+                            }
                             uint32_t k0p[SC];
                             load_meta<SC>(sm.meta, stage, cl, k0p);
                             const uint32_t slots_u32 = stage_u32 + (cl * SC) * SG::bytes;
@@ -1412,7 +1470,10 @@ __global__ void __launch_bounds__(kStThreads, SC >= 8 ? 2 : 3) das_staged2_kerne
                                 acc2 = __ffma2_rn(w2[j], make_float2(ta, tb), acc2);
                             }
                         }
-                    } else {
+                        };
+                        if (p.srcdir) channels(std::true_type{});
+                        else channels(std::false_type{});
+                    } else {   // a window wider than its slot: its taps read the pair rows
 #pragma unroll 1
                     for (int cl = 0; cl < CC; cl++) {
                         const int c = c0 + cl;
@@ -1435,46 +1496,28 @@ __global__ void __launch_bounds__(kStThreads, SC >= 8 ? 2 : 3) das_staged2_kerne
                             apply_directivity(ga, cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z, dir);
                             apply_directivity(gb, cx.vx2, cx.vy2, cx.vz2, cp.x, cp.y, cp.z, dir);
                         }
-                        const float2 rsq2 = make_float2(ga.rsq, gb.rsq), rinv2 = make_float2(ga.rinv, gb.rinv);
                         uint32_t k0p[SC];
                         load_meta<SC>(sm.meta, stage, cl, k0p);
-                        const uint32_t slots_u32 = stage_u32 + (cl * SC) * SG::bytes;
-                        if (!any_ovf) {
+                        const unsigned char *slots = sm.ring + stage * SG::stage_bytes + (cl * SC) * SG::bytes;
 #pragma unroll
-                            for (int j = 0; j < SC; j++) {
-                                const float2 tau2 = __ffma2_rn(rsq2, rinv2, ofs2[j]);
-                                const float2 mm2 = __fadd2_rd(tau2, magic2);
-                                const float2 nfl2 = __ffma2_rn(mm2, neg1, magic2);   // -(floor), exact
-                                const float2 t2 = __fadd2_rn(tau2, nfl2);
-                                const uint32_t ra = min(__float_as_uint(mm2.x) - k0p[j], (uint32_t)WB);
-                                const uint32_t rb = min(__float_as_uint(mm2.y) - k0p[j], (uint32_t)WB);
-                                const uint32_t slot = slots_u32 + j * SG::bytes;
-                                const float ta = tap_at<K>(slot + ra * sizeof(st), t2.x);
-                                const float tb = tap_at<K>(slot + rb * sizeof(st), t2.y);
-                                acc2 = __ffma2_rn(w2[j], make_float2(ta, tb), acc2);
-                            }
-                        } else {
-                            const unsigned char *slots = sm.ring + stage * SG::stage_bytes + (cl * SC) * SG::bytes;
+                        for (int j = 0; j < SC; j++) {
+                            float tv[2];
 #pragma unroll
-                            for (int j = 0; j < SC; j++) {
-                                float tv[2];
-#pragma unroll
-                                for (int h = 0; h < 2; h++) {
-                                    const recv_geom &g = h ? gb : ga;
-                                    const float tau = __fmaf_rn(g.rsq, g.rinv, h ? ofs2[j].y : ofs2[j].x);
-                                    const tau_split ts = split_tau(tau);
-                                    st pr;
-                                    if (k0p[j] == kOvf) {
-                                        const int64_t row = ((int64_t)cx.b * p.C + c) * p.S + (e0 + min(j, sc - 1));
-                                        pr = Pg[row * p.npad + min(ts.k, kmax_pair)];
-                                    } else {
-                                        const uint32_t rel = min(ts.k + kFloorMagicBits - k0p[j], (uint32_t)WB);
-                                        pr = *reinterpret_cast<const st *>(slots + j * SG::bytes + rel * sizeof(st));
-                                    }
-                                    tv[h] = pair_traits<K>::tap(pr, ts.t);
+                            for (int h = 0; h < 2; h++) {
+                                const recv_geom &g = h ? gb : ga;
+                                const float tau = __fmaf_rn(g.rsq, g.rinv, h ? ofs2[j].y : ofs2[j].x);
+                                const tau_split ts = split_tau(tau);
+                                st pr;
+                                if (k0p[j] == kOvf) {
+                                    const int64_t row = ((int64_t)cx.b * p.C + c) * p.S + (e0 + min(j, sc - 1));
+                                    pr = Pg[row * p.npad + min(ts.k, kmax_pair)];
+                                } else {
+                                    const uint32_t rel = min(ts.k + kFloorMagicBits - k0p[j], (uint32_t)WB);
+                                    pr = *reinterpret_cast<const st *>(slots + j * SG::bytes + rel * sizeof(st));
                                 }
-                                acc2 = __ffma2_rn(w2[j], make_float2(tv[0], tv[1]), acc2);
+                                tv[h] = pair_traits<K>::tap(pr, ts.t);
                             }
+                            acc2 = __ffma2_rn(w2[j], make_float2(tv[0], tv[1]), acc2);
                         }
                     }
                     }
@@ -1594,6 +1637,8 @@ constexpr size_t staged_batch_smem_bytes() {
 template <int K, int SC, int WB, int BT>
 __global__ void __launch_bounds__(kStThreads) das_staged_batch_kernel(const staged_params p,
                                                                        const __grid_constant__ CUtensorMap tmap) {
+    tile_shape shape;
+    if (!take_plan<WB, true>(p, shape)) return;
     using st = typename pair_traits<K>::storage;
     using SG = slot_geom<WB, K>;
     using GG = group_geom<WB, K, BT>;
@@ -1604,7 +1649,7 @@ __global__ void __launch_bounds__(kStThreads) das_staged_batch_kernel(const stag
     staged_smem<K, WB> sm(smem_raw);
     unsigned char *zero_group = sm.extra;
     for (int i = threadIdx.x; i < GG::data_bytes / 4; i += kStThreads) reinterpret_cast<uint32_t *>(zero_group)[i] = 0u;
-    const staged_ctx cx = staged_setup<K, WB>(p, sm);   // ends with __syncthreads
+    const staged_ctx cx = staged_setup<K, WB, true, true>(p, shape, sm);   // ends with __syncthreads
 
     const st *__restrict__ Pg = static_cast<const st *>(p.P);
     const uint32_t kmax_pair = (uint32_t)(p.npad - 1);
@@ -1756,8 +1801,14 @@ __global__ void __launch_bounds__(kStThreads) das_staged_batch_kernel(const stag
 // added once per channel per CTA.  Voxels are spread over the warps
 // (staged_setup's spread mapping) so a warp's lanes rarely share a sample.
 template <int K, int SC, int WB>
-__global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_kernel(const staged_params p,
+__global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_kernel(const staged_params params,
                                                                      const __grid_constant__ CUtensorMap tmap) {
+    staged_params p = params;   // (as das_staged2_kernel)
+    {
+        tile_shape shape;
+        if (!take_plan<WB>(p, shape)) return;
+        p.T0 = shape.T0; p.T1 = shape.T1; p.T2 = shape.T2; p.n0 = shape.n0; p.n1 = shape.n1;
+    }
     using SG = slot_geom<WB, K>;
     using st = typename pair_traits<K>::storage;
     constexpr int CC = kStWin / SC;
@@ -1774,7 +1825,7 @@ __global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_kernel(const sta
     float *cgrad = reinterpret_cast<float *>(gslot + kBinCopies * kRegion);  // [CC * 3][256]
     float *wmax = cgrad + CC * 3 * kStConsumers;                          // [kStWarps]
     for (int i = threadIdx.x; i < kBinCopies * kRegion; i += kStThreads) gslot[i] = 0;
-    const staged_ctx cx = staged_setup<K, WB>(p, sm, true);   // ends with __syncthreads
+    const staged_ctx cx = staged_setup<K, WB>(p, tile_shape{p.T0, p.T1, p.T2, p.n0, p.n1}, sm, true);   // ends with __syncthreads
     const uint32_t gslot_u32 = smem_u32(gslot) + cx.par * (kRegion * 4);   // this thread's copy
 
     const bool multi_b = p.B > 1 || gridDim.z > 1;   // several CTAs add into the voxel-side gradients
@@ -2058,8 +2109,14 @@ constexpr size_t staged_bwd_batch_smem_bytes() {
 }
 
 template <int K, int SC, int WB, int BT>
-__global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_batch_kernel(const staged_params p,
+__global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_batch_kernel(const staged_params params,
                                                                             const __grid_constant__ CUtensorMap tmap) {
+    staged_params p = params;   // (as das_staged2_kernel)
+    {
+        tile_shape shape;
+        if (!take_plan<WB>(p, shape)) return;
+        p.T0 = shape.T0; p.T1 = shape.T1; p.T2 = shape.T2; p.n0 = shape.n0; p.n1 = shape.n1;
+    }
     using SG = slot_geom<WB, K>;
     using GG = group_geom<WB, K, BT>;
     using st = typename pair_traits<K>::storage;
@@ -2088,7 +2145,7 @@ __global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_batch_kernel(con
     unsigned char *zero_group = sm.extra + kZeroOff;
     for (int i = threadIdx.x; i < 2 * kSet; i += kStThreads) gslot[i] = 0;
     for (int i = threadIdx.x; i < GG::data_bytes / 4; i += kStThreads) reinterpret_cast<uint32_t *>(zero_group)[i] = 0u;
-    const staged_ctx cx = staged_setup<K, WB>(p, sm, true);   // ends with __syncthreads
+    const staged_ctx cx = staged_setup<K, WB>(p, tile_shape{p.T0, p.T1, p.T2, p.n0, p.n1}, sm, true);   // ends with __syncthreads
     const uint32_t gslot_u32 = smem_u32(gslot) + cx.par * (kRegion * 4);   // this thread's copy
     const uint32_t zero_u32 = smem_u32(zero_group);
 
@@ -2423,7 +2480,7 @@ __global__ void __launch_bounds__(kStThreads) das_staged_cplx_kernel(const stage
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     staged_smem<K, WB> sm(smem_raw);
-    const staged_ctx cx = staged_setup<K, WB>(p, sm);
+    const staged_ctx cx = staged_setup<K, WB>(p, tile_shape{p.T0, p.T1, p.T2, p.n0, p.n1}, sm);
     const int cbeg = chan_begin(p), cend = chan_end(p);
     const st *__restrict__ Pg = static_cast<const st *>(p.P);
     const uint32_t kmax_pair = (uint32_t)(p.npad - 1);
@@ -2516,7 +2573,7 @@ __global__ void __launch_bounds__(kStThreads) das_staged_cplx_kernel(const stage
 
 // Prepares the image for channel slices that add into it: out = beta * out
 // (or 0) for every batch item and voxel.
-__global__ void __launch_bounds__(256) scale_image_kernel(float *out, int64_t bstride, int64_t V, int B,
+static __global__ void __launch_bounds__(256) scale_image_kernel(float *out, int64_t bstride, int64_t V, int B,
                                                           float beta, int beta_zero, const int *gate) {
     if (gate && *(volatile const int *)gate) return;   // the staged call is off: the gather kernel applies beta
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

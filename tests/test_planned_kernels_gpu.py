@@ -1,0 +1,90 @@
+"""GPU tests of the kernels a call without a schedule takes: the staged kernels
+on a planned tile shape, IQ batch tiles, sorted list entries and the tensor-core
+batches, at sizes where they can go wrong (ragged tiles, windows wider than a
+slot, record ends, channel remainders), against the FP64 oracle and the float64
+torch reference.
+
+Tolerances: an image is a sum of taps whose delays are rounded to FP32, a
+relative error of about 2^-23 N * 0.25 cycles * 2 pi per tap on this white data
+(3e-5 at N = 600 measured for every kernel), so 1e-4 holds each case.  A delay
+rounded across a sample boundary takes the neighbouring slope: with |d tau| up
+to 6e-5 a share 2 |d tau| of the taps does, each off by about 1.6 of its own size,
+so delay and position gradients are held to sqrt(1.2e-4) * 1.6 = 1.8e-2, to 2.5e-2.
+"""
+import numpy as np
+import pytest
+import torch
+
+import ffdas_b200
+from oracle import oracle
+from torch_ref import das_ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+TOL = 1e-4
+GTOL = 2.5e-2
+
+
+def _problem(B, C, S, N, nz, nx, pitch=(1.0, 1.0), dtype=torch.float32, seed=0, n=None, z0=20.0):
+    """Linear array, (nz, nx) pixels `pitch` wavelengths apart, delays within the record and past both its ends."""
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn((B, C, S, N), generator=g, dtype=torch.complex64 if dtype.is_complex else torch.float32)
+    src = torch.zeros((C, 3))
+    src[:, 0] = torch.arange(C) - (C - 1) / 2
+    z = z0 + pitch[0] * torch.arange(nz, dtype=torch.float32)
+    xx = pitch[1] * (torch.arange(nx, dtype=torch.float32) - (nx - 1) / 2)
+    zz, xg = torch.meshgrid(z, xx, indexing="ij")
+    dst = torch.stack([xg, 0.1 * xg, zz], -1).contiguous()
+    E = S if n is None else n
+    offs = (zz[None] + 0.3 * torch.arange(E)[:, None, None] * xg / max(nx, 1) - z0 - 3.0).contiguous()
+    w = (torch.rand((E, nz, nx), generator=g) + 0.2)
+    return x.to(dtype), src, dst, offs, w
+
+
+def _dev(*ts):
+    return [t.to(DEV) for t in ts]
+
+
+def _info():
+    return ffdas_b200.get_library_handle(torch.device(DEV)).last_kernel_info()
+
+
+def _oracle(x, src, dst, offs, w, **kw):
+    xn = x.to(torch.complex64 if x.is_complex() else torch.float32).numpy()
+    kw = {k: (v.numpy() if torch.is_tensor(v) else v) for k, v in kw.items()}
+    return oracle.das_f64(xn, src.numpy(), dst.numpy(), offs.numpy(), w.numpy(), **kw)
+
+
+def _cone(C):
+    d = torch.zeros((C, 4))
+    d[:, 2], d[:, 3] = 1.0, 0.81
+    return d
+
+
+@pytest.mark.parametrize("pitch", [(0.2, 0.2), (1.7, 0.5), (5.0, 0.4), (0.3, 6.0)], ids=str)
+@pytest.mark.parametrize("B,S", [(1, 1), (1, 5), (3, 4)])
+@pytest.mark.parametrize("cone", [False, True])
+def test_planned_tiles(pitch, B, S, cone):
+    # 131 x 67 pixels and 41 channels divide no tile or stage; fine, ordinary and
+    # coarse pitches along either axis take different shapes and widths
+    x, src, dst, offs, w = _problem(B, 41, S, 600, 131, 67, pitch, seed=S)
+    rep = 30 if S > 1 else 120               # enough channels to pass the direct kernel's range
+    big = torch.cat([x] * rep, dim=1), src.repeat(rep, 1)
+    srcdir = _cone(41 * rep) if cone else None
+    got = ffdas_b200.das(*_dev(big[0], big[1], dst, offs, w), srcdir=srcdir.to(DEV) if cone else None)
+    assert _info()["variant"] == 2
+    ref = rep * _oracle(x, src, dst, offs, w, srcdir=_cone(41) if cone else None)
+    assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL
+
+
+@pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9, 16, 17, 31, 32])
+@pytest.mark.parametrize("S", [33, 97])
+def test_select_sizes(k, S):
+    # around the group sizes 4, 8, 16, 32 and the staged event limit, one voxel past a block
+    g = torch.Generator().manual_seed(k * 100 + S)
+    w = torch.randint(0, 9, (S, 129), generator=g).float()      # many ties
+    o = torch.rand((S, 129), generator=g)
+    idx, sw, so = ffdas_b200.sparse_select(w.to(DEV), k, offsets=o.to(DEV))
+    order = torch.sort(w, dim=0, descending=True, stable=True)[1][:k]
+    assert torch.equal(idx.cpu().long(), order)
+    assert torch.equal(sw.cpu(), w.gather(0, order)) and torch.equal(so.cpu(), o.gather(0, order))
