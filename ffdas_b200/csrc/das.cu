@@ -535,6 +535,29 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         }
     }
 
+    // ---- dense complex (IQ) data without a schedule: batch tiles on windows of
+    // plain samples (das_iq.cuh).  (A pair buffer stays unfilled: its adjoint
+    // reads no pairs.)
+    if (!h.has_config && od.dtype == FFDAS_C_32F && iq_supported(pb, kind)) {
+        const float *gain = nullptr;
+        int gain_bstride = 0;
+        FFDAS_TRY(channel_gain(h, pb, &gain, &gain_bstride));
+        workspace IW(h);
+        FFDAS_TRY(IW.alloc(iq_workspace(pb, xd.dtype, kind, a.x, gain)));
+        gather_params gp;
+        std::memset(&gp, 0, sizeof(gp));
+        gp.C = pb.C; gp.S = pb.S; gp.n_events = pb.n_events; gp.B = pb.B; gp.V = pb.V;
+        gp.D0 = pb.D0; gp.D1 = pb.D1; gp.D2 = pb.D2;
+        gp.srcpos = a.srcpos; gp.srcdir = reinterpret_cast<const float4 *>(a.srcdir);
+        gp.dstpos = a.dstpos; gp.offsets = a.offsets; gp.weights = a.weights;
+        gp.wavenum = a.wavenum;
+        gp.out = a.out;
+        gp.out_bstride = pb.out_bstride;
+        read_beta(od.dtype, a.beta, gp.beta_re, gp.beta_im, gp.beta_zero);
+        h.last = ffdas_kernel_info_t{};
+        return launch_iq(h, pb, xd.dtype, kind, a.x, gain, gain_bstride, gp, IW.get<void>());
+    }
+
     // ---- ingest: x -> pair rows (workspace) ----
     const int64_t npad = pair_row_length(pb.N);
     const int64_t rows = (int64_t)pb.B * pb.C * pb.S;

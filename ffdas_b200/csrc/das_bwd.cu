@@ -770,6 +770,24 @@ ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tens
     if (!gx && !goff && !gw && !gdst && !gsrc) return FFDAS_SUCCESS;
 
     pb.sparse = a.sparse;
+    // dense complex data without a schedule: staged sample windows, shared-memory bins
+    if (cplx && !h.has_config && iq_supported(pb, kind)) {
+        workspace IW(h);
+        FFDAS_TRY(IW.alloc(iq_workspace(pb, xd.dtype, kind, a.x, nullptr)));
+        gather_params gp;
+        std::memset(&gp, 0, sizeof(gp));
+        gp.C = pb.C; gp.S = pb.S; gp.n_events = pb.n_events; gp.B = pb.B; gp.V = pb.V;
+        gp.D0 = pb.D0; gp.D1 = pb.D1; gp.D2 = pb.D2;
+        gp.srcpos = a.srcpos; gp.srcdir = reinterpret_cast<const float4 *>(a.srcdir);
+        gp.dstpos = a.dstpos; gp.offsets = a.offsets; gp.weights = a.weights;
+        gp.wavenum = a.wavenum;
+        gp.beta_zero = 1;
+        const staged_grads gr{static_cast<const float *>(gout), pb.out_bstride, gx, goff, gw, gdst, gsrc};
+        h.last = ffdas_kernel_info_t{};
+        h.last_pairs_reused = false;
+        return launch_iq_bwd(h, pb, xd.dtype, kind, a.x, gp, gr, IW.get<void>());
+    }
+
     const int64_t npad = pair_row_length(pb.N);
     const int64_t rows = (int64_t)pb.B * pb.C * pb.S;
     const size_t sb = kind == ST_C32 ? 16 : (kind == ST_F32 || kind == ST_C16) ? 8 : 4;

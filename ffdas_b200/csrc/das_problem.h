@@ -104,6 +104,14 @@ struct staged_grads {
     int64_t gout_bstride;
     float *gx, *goff, *gw, *gdst, *gsrc;
 };
+// Dense complex (IQ) data on batch tiles of sample windows (das_iq.cuh), FP32 or
+// FP16 samples; ws is iq_workspace() bytes; gr holds float views of the gradients.
+bool iq_supported(const das_problem &pb, int kind);
+size_t iq_workspace(const das_problem &pb, ffdas_datatype_t xt, int kind, const void *x, const float *gain);
+ffdas_error_t launch_iq(ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt, int kind, const void *x,
+                        const float *gain, int gain_bstride, gather_params gp, void *ws);
+ffdas_error_t launch_iq_bwd(ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt, int kind, const void *x,
+                            gather_params gp, const staged_grads &gr, void *ws);
 // Zeroes the given gradient outputs (null: none) in one launch: gw and goff of
 // list_n floats, gdst of dst_n, gsrc of src_n.
 ffdas_error_t clear_gradients(ffdas_context &h, float *gw, float *goff, int64_t list_n, float *gdst, int64_t dst_n,

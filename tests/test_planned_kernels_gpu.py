@@ -77,6 +77,53 @@ def test_planned_tiles(pitch, B, S, cone):
     assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL
 
 
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex32])
+@pytest.mark.parametrize("B,S,C,N", [(1, 1, 24, 500), (1, 4, 17, 40), (2, 5, 33, 501), (3, 3, 9, 502), (4, 2, 30, 96), (5, 8, 40, 500)])
+@pytest.mark.parametrize("pitch", [(0.7, 0.5), (6.0, 0.5)], ids=str)
+def test_iq_batch_tiles(dtype, B, S, C, N, pitch):
+    # rows read in place and copied (odd lengths), shorter than a window, one to four items a tile
+    x, src, dst, offs, w = _problem(B, C, S, N, 50, 37, pitch, dtype=torch.complex64, seed=B + S)
+    x = x.to(dtype)
+    wn = -1.3
+    got = ffdas_b200.das(*_dev(x, src, dst, offs, w), srcdir=_cone(C).to(DEV), wavenum=wn)
+    assert _info()["variant"] == 2 and got.dtype == torch.complex64
+    ref = _oracle(x, src, dst, offs, w, srcdir=_cone(C), wavenum=wn)
+    assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL * (1 + abs(wn))
+
+
+def test_iq_strided_data():
+    # channels trailing, a row pitch of its own, and starts that are not 16-byte aligned
+    x, src, dst, offs, w = _problem(3, 20, 4, 300, 50, 37, dtype=torch.complex64)
+    args = _dev(src, dst, offs, w)
+    ref = ffdas_b200.das(x.to(DEV), *args, wavenum=0.3)
+    wide = torch.zeros((3, 20, 4, 330), device=DEV, dtype=torch.complex64)
+    for first in (0, 8, 3):
+        wide[..., first:first + 300] = x.to(DEV)
+        got = ffdas_b200.das(wide[..., first:first + 300], *args, wavenum=0.3)   # sums in another order at most
+        assert torch.linalg.norm(got - ref) < 1e-6 * torch.linalg.norm(ref)
+    xt = x.transpose(1, 2).contiguous().to(DEV)
+    got = ffdas_b200.das(xt, *args, wavenum=0.3, channels_trailing=True)
+    assert torch.linalg.norm(got - ref) < 1e-6 * torch.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("B,S,C,N,pitch", [(1, 1, 9, 300, (0.7, 0.5)), (2, 5, 20, 301, (0.7, 0.5)), (3, 4, 40, 300, (0.6, 4.0)),
+                                           (2, 3, 12, 299, (9.0, 0.5)), (4, 1, 70, 48, (0.3, 0.3)), (6, 6, 13, 128, (0.7, 0.5))], ids=str)
+def test_iq_adjoint(B, S, C, N, pitch):
+    x, src, dst, offs, w = _problem(B, C, S, N, 24, 19, pitch, dtype=torch.complex64, seed=3)
+    wn = 0.4
+    gpu = [t.to(DEV).requires_grad_(True) for t in (x, src, dst, offs, w)]
+    ref = [t.to(torch.complex128 if t.is_complex() else torch.float64).requires_grad_(True)
+           for t in (x, src, dst, offs, w)]
+    g = torch.Generator().manual_seed(1)
+    gy = torch.randn((B, 24, 19), generator=g, dtype=torch.complex64)
+    ffdas_b200.das(*gpu, wavenum=wn).backward(gy.to(DEV))
+    assert _info()["variant"] == 8
+    das_ref(*ref, wavenum=wn).backward(gy.to(torch.complex128))
+    for name, a, b in zip(("x", "srcpos", "dstpos", "offsets", "weights"), gpu, ref):
+        tol = TOL if name in ("x", "weights") else GTOL
+        assert oracle.rel_l2(a.grad.cpu().numpy(), b.grad.numpy()) < tol, name
+
+
 @pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9, 16, 17, 31, 32])
 @pytest.mark.parametrize("S", [33, 97])
 def test_select_sizes(k, S):
