@@ -535,6 +535,15 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         }
     }
 
+    // ---- large half-precision batches: tensor cores, straight from x ----
+    // (not with a pair buffer to fill, a channel scale or a prior image to keep)
+    if (!h.has_config && !h.chan_scale && !h.pair_buf && mma_supported(pb, xd.dtype, od.dtype, kind)) {
+        double br = 0.0, bi = 0.0;
+        int bz = 1;
+        read_beta(od.dtype, a.beta, br, bi, bz);
+        if (bz) return launch_mma(h, pb, a, static_cast<float *>(a.out));
+    }
+
     // ---- dense complex (IQ) data without a schedule: batch tiles on windows of
     // plain samples (das_iq.cuh).  (A pair buffer stays unfilled: its adjoint
     // reads no pairs.)

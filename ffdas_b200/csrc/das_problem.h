@@ -127,6 +127,11 @@ ffdas_error_t launch_staged_sparse(ffdas_context &h, const das_problem &pb, int 
 ffdas_error_t launch_staged_bwd(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp,
                                 const staged_grads &gr, int SC, int WB, int BT, int copy, dim3 grid);
 
+// Large half-precision batches on the tensor cores (csrc/das_mma.cuh), straight
+// from x: half data at its default precision, FP32 output, beta 0.
+bool mma_supported(const das_problem &pb, ffdas_datatype_t xt, ffdas_datatype_t ot, int kind);
+ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call &a, float *out);
+
 // das_sparse as one persistent launch over (tile, channel slice) work items,
 // longest tiles first (csrc/das_sparse_items.cuh): real pair storage, f32
 // output, lists of at most 64 entries.  gp holds 256-voxel tiles and the

@@ -124,6 +124,39 @@ def test_iq_adjoint(B, S, C, N, pitch):
         assert oracle.rel_l2(a.grad.cpu().numpy(), b.grad.numpy()) < tol, name
 
 
+@pytest.mark.parametrize("B,C,S,N,pitch", [(32, 9, 1, 256, (1.0, 0.5)), (33, 40, 3, 250, (1.5, 0.5)), (64, 17, 4, 504, (6.0, 0.5)),
+                                           (270, 8, 2, 160, (0.5, 0.5))], ids=str)
+def test_tensor_core_batches(B, C, S, N, pitch):
+    # item counts off the multiples of 16 and past one product's 256 columns,
+    # rows that are not 16-byte aligned, windows wider than one box, weights
+    # spread over six decades (hi + lo parts under one scale per voxel)
+    x, src, dst, offs, w = _problem(B, C, S, N, 37, 29, pitch, dtype=torch.float16, seed=B)
+    w = w * 10.0 ** (-6.0 * torch.rand(w.shape, generator=torch.Generator().manual_seed(7)))
+    for srcdir in (None, _cone(C)):
+        got = ffdas_b200.das(*_dev(x, src, dst, offs, w), srcdir=None if srcdir is None else srcdir.to(DEV))
+        assert _info()["variant"] == 10
+        ref = _oracle(x, src, dst, offs, w, srcdir=srcdir)
+        assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL
+
+
+def test_tensor_core_batches_channels_trailing_view_and_non_finite_values():
+    # a (B, S, C, N) view; an infinite and a NaN sample, a NaN delay and an
+    # infinite weight reach the values whose taps meet them and no others
+    x, src, dst, offs, w = _problem(40, 12, 3, 256, 40, 31, (1.0, 0.5), dtype=torch.float16, seed=5)
+    clean = _oracle(x, src, dst, offs, w)
+    x[3, 4, 1, 100], x[7, 2, 0, 60] = float("inf"), float("nan")
+    offs[1, 5, 5], w[2, 30, 8] = float("nan"), float("inf")
+    ref = _oracle(x, src, dst, offs, w)
+    ref[:, 5, 5] = np.nan   # a NaN delay makes its voxel NaN; the oracle leaves the tap out
+    xt = x.transpose(1, 2).contiguous().to(DEV)
+    got = ffdas_b200.das(xt, *_dev(src, dst, offs, w), channels_trailing=True).cpu().numpy()
+    assert _info()["variant"] == 10
+    assert (np.isfinite(got) == np.isfinite(ref)).mean() > 0.9999   # a delay may round across a spoiled sample
+    both = np.isfinite(got) & np.isfinite(ref)
+    assert both.mean() > 0.9 and not both.all()
+    assert oracle.rel_l2(got[both], clean[both]) < TOL
+
+
 @pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9, 16, 17, 31, 32])
 @pytest.mark.parametrize("S", [33, 97])
 def test_select_sizes(k, S):
