@@ -12,13 +12,14 @@ dtype and layout.
 """
 from __future__ import annotations
 
-import ctypes
+from array import array
 
 import torch
 
 from . import _lib
 from ._lib import DataType
-from .das import _FFDAS_DTYPE, _astype, _check_spatial, _compute_type, _run, _to_torch, _x_desc
+from .das import (_FFDAS_DTYPE, _astype, _bits, _check_spatial, _compute_type, _raw_stream, _run, _to_torch, _x_desc,
+                  _x_layout)
 from .library import get_library_handle
 
 
@@ -34,23 +35,18 @@ class DASFunction(torch.autograd.Function):
         ctx.opts = opts
         ctx.pairs = None
         xt = x.detach()
-        handle = get_library_handle(xt.device)
         # The forward builds its interpolation-pair rows into a buffer kept for
         # the backward (ffdas_set_pair_buffer), which then skips building them
         # again; only where the backward can run.
-        keep = _backward_supported(xt, opts["wavenum"])
-        if keep:
+        pair_buffer = None
+        if _backward_supported(xt, opts["wavenum"]):
             nbytes = _lib.pair_bytes(_x_desc(xt, opts["channels_trailing"]), _compute_type(xt, False, False))
             ctx.pairs = torch.empty(nbytes, dtype=torch.uint8, device=xt.device)
-            handle.set_pair_buffer(ctx.pairs.data_ptr(), nbytes)
-        try:
-            out = _run(xt, srcpos.detach(), dstpos.detach(), offsets.detach(), weights.detach(),
-                       sparse_indices, srcdir=opts["srcdir"], wavenum=opts["wavenum"], algorithm=0,
-                       use_fp16=opts["use_fp16"], use_bf16=opts["use_bf16"],
-                       channels_trailing=opts["channels_trailing"], out=None)
-        finally:
-            if keep:
-                handle.set_pair_buffer(None, 0)
+            pair_buffer = (ctx.pairs.data_ptr(), nbytes)
+        out = _run(xt, srcpos.detach(), dstpos.detach(), offsets.detach(), weights.detach(), sparse_indices,
+                   srcdir=opts["srcdir"], wavenum=opts["wavenum"], algorithm=0, use_fp16=opts["use_fp16"],
+                   use_bf16=opts["use_bf16"], channels_trailing=opts["channels_trailing"], out=None,
+                   pair_buffer=pair_buffer)
         ctx.save_for_backward(x, srcpos, dstpos, offsets, weights,
                               sparse_indices if sparse_indices is not None else torch.empty(0))
         ctx.has_sparse = sparse_indices is not None
@@ -79,32 +75,21 @@ class DASFunction(torch.autograd.Function):
         gdst = torch.empty(dstpos.shape, dtype=torch.float32, device=dev) if need[2] else None
         gsrc = torch.empty(srcpos.shape, dtype=torch.float32, device=dev) if need[1] else None
 
-        dims = list(xt.shape)
-        strides = list(xt.stride())
-        if opts["channels_trailing"]:
-            c = 1 if xt.ndim == 4 else 0
-            dims[c], dims[c + 1] = dims[c + 1], dims[c]
-            strides[c], strides[c + 1] = strides[c + 1], strides[c]
-        x_desc = _lib.TensorDesc(dims, strides, _FFDAS_DTYPE[xt.dtype])
-        g_desc = _lib.TensorDesc(list(gout.shape), list(gout.stride()), DataType.C_32F if cplx else DataType.R_32F)
         f32 = lambda t: _astype(t.detach(), torch.float32, dev, "input")  # noqa: E731
         srcpos_t, dstpos_t, offsets_t, weights_t = f32(srcpos), f32(dstpos), f32(offsets), f32(weights)
         srcdir_t = f32(_to_torch(opts["srcdir"])) if opts["srcdir"] is not None else None
         idx_t = _astype(idx, torch.int32, dev, "sparse_indices") if ctx.has_sparse else None
         handle = get_library_handle(dev)
-        handle.set_stream(torch.cuda.current_stream(dev).cuda_stream)
-        ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
-        if ctx.pairs is not None:   # the forward's pair rows, read instead of rebuilt when they match
-            handle.set_pair_buffer(ctx.pairs.data_ptr(), ctx.pairs.numel())
-        try:
-            _lib.check(_lib.load().ffdas_das_backward(
-                handle.h, ptr(srcpos_t), ptr(srcdir_t), float(opts["wavenum"]), x_desc.desc, ptr(xt), ptr(dstpos_t),
-                ptr(offsets_t),
-                ptr(weights_t), int(idx_t.shape[0]) if idx_t is not None else 0, ptr(idx_t), g_desc.desc,
-                ptr(gout), ptr(gx), ptr(goff), ptr(gw), ptr(gdst), ptr(gsrc)))
-        finally:
-            if ctx.pairs is not None:
-                handle.set_pair_buffer(None, 0)
+        ptr = lambda t: 0 if t is None else t.data_ptr()  # noqa: E731
+        # one native call; the forward's pair rows are read instead of rebuilt when they match
+        gd = gout.shape
+        q = array("q", [handle.h.value, _raw_stream(dev.index), ptr(srcpos_t), ptr(srcdir_t), _bits(opts["wavenum"]),
+                        ptr(xt), _FFDAS_DTYPE[xt.dtype], *_x_layout(xt, opts["channels_trailing"]), ptr(dstpos_t),
+                        ptr(offsets_t), ptr(weights_t), idx_t.shape[0] if idx_t is not None else 0, ptr(idx_t),
+                        ptr(gout), DataType.C_32F if cplx else DataType.R_32F, ptr(gx), ptr(goff), ptr(gw), ptr(gdst),
+                        ptr(gsrc), ptr(ctx.pairs), ctx.pairs.numel() if ctx.pairs is not None else 0, len(gd), *gd,
+                        *gout.stride()])
+        _lib.check(_lib.load().ffdas_das_backward_call(q.buffer_info()[0], len(q)))
         ctx.pairs = None
         if gx is not None:
             if opts["channels_trailing"]:

@@ -30,8 +30,10 @@ Differences from the reference (documented, deliberate):
 from __future__ import annotations
 
 import ctypes
+import struct
 import sys
 import warnings
+from array import array
 
 import torch
 
@@ -67,7 +69,7 @@ _OUT_DTYPE = {
 
 
 def _shape(a):
-    return tuple(a.shape)
+    return a.shape if type(a) is torch.Tensor else tuple(a.shape)   # torch.Size is a tuple
 
 
 def _to_torch(a):
@@ -102,7 +104,29 @@ def _astype(a, dtype: torch.dtype, device, name: str, stacklevel: int = 4):
         t = t.to(dtype)
     if t.device != device:
         raise ValueError(f"{name} is on {t.device}, expected {device}")
-    return t.contiguous()
+    return t if t.is_contiguous() else t.contiguous()
+
+
+def _raw_stream(index: int) -> int:
+    """cudaStream_t of torch's current stream on a device."""
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
+def _x_layout(x: torch.Tensor, channels_trailing: bool):
+    """ndim, four dims and four strides of x as ([batch,] channels, sequence, samples), padded with 0."""
+    dims, strides = list(x.shape), list(x.stride())
+    n = len(dims)
+    if channels_trailing:
+        # reference _ffdas.cpp:515-519: swap the channel and sequence dims
+        c = n - 3
+        dims[c], dims[c + 1] = dims[c + 1], dims[c]
+        strides[c], strides[c + 1] = strides[c + 1], strides[c]
+    pad = [0] * (4 - n)
+    return [n, *dims, *pad, *strides, *pad]
+
+
+def _bits(f: float) -> int:
+    return struct.unpack("<q", struct.pack("<d", f))[0]   # a double's bits, for an int64 argument array
 
 
 def _compute_type(x: torch.Tensor, use_fp16: bool, use_bf16: bool) -> ComputeType:
@@ -135,17 +159,18 @@ def _beta_buffer(dtype: torch.dtype):
 
 
 def _check_spatial(dstpos, offsets, weights, sparse_indices=None):
-    if len(_shape(dstpos)) < 2 or _shape(dstpos)[-1] != 3:
+    ds = _shape(dstpos)
+    if len(ds) < 2 or ds[-1] != 3:
         raise ValueError("dstpos must have dimensions (..., 3)")
-    spatial = _shape(dstpos)[:-1]
+    spatial = ds[:-1]
     if _shape(offsets)[1:] != spatial:
-        raise ValueError(f"offsets shape {_shape(offsets)} must match target layout {spatial}")
+        raise ValueError(f"offsets shape {tuple(offsets.shape)} must match target layout {tuple(spatial)}")
     if _shape(weights)[1:] != spatial:
-        raise ValueError(f"weights shape {_shape(weights)} must match target layout {spatial}")
+        raise ValueError(f"weights shape {tuple(weights.shape)} must match target layout {tuple(spatial)}")
     if sparse_indices is not None:
         if _shape(sparse_indices)[1:] != spatial:
-            raise ValueError(
-                f"sparse_indices shape {_shape(sparse_indices)} must match target layout {spatial}")
+            raise ValueError(f"sparse_indices shape {tuple(sparse_indices.shape)} must match target layout "
+                             f"{tuple(spatial)}")
         n = _shape(sparse_indices)[0]
         if _shape(offsets)[0] != n or _shape(weights)[0] != n:
             raise ValueError(f"offsets and weights leading dimension must match sparse count {n}")
@@ -157,7 +182,7 @@ def _needs_grad(*ts) -> bool:
 
 
 def _run(x, srcpos, dstpos, offsets, weights, sparse_indices, *, srcdir, wavenum, algorithm,
-         use_fp16, use_bf16, channels_trailing, out, channel_scale=None, host_chunks=None):
+         use_fp16, use_bf16, channels_trailing, out, channel_scale=None, host_chunks=None, pair_buffer=None):
     spatial = _check_spatial(dstpos, offsets, weights, sparse_indices)
     xt = _to_torch(x)
     if xt.ndim not in (3, 4):
@@ -191,16 +216,7 @@ def _run(x, srcpos, dstpos, offsets, weights, sparse_indices, *, srcdir, wavenum
         out_t = torch.empty(out_dims, dtype=out_dtype, device=dev)
     else:
         out_t = _to_torch(out)
-    beta = _beta_buffer(out_t.dtype)
     ctype = _compute_type(xt, use_fp16, use_bf16)
-
-    handle = get_library_handle(dev)
-    handle.set_stream(torch.cuda.current_stream(dev).cuda_stream)
-    x_desc = _x_desc(xt, channels_trailing)
-    o_desc = _lib.TensorDesc(list(out_t.shape), list(out_t.stride()),
-                             _FFDAS_DTYPE.get(out_t.dtype, DataType.R_32F))
-    L = _lib.load()
-    ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
     scale_t = None
     if channel_scale is not None:
         scale_t = _astype(channel_scale, torch.float32, dev, "channel_scale")
@@ -209,22 +225,37 @@ def _run(x, srcpos, dstpos, offsets, weights, sparse_indices, *, srcdir, wavenum
         if scale_t.numel() not in (C, B * C):
             raise ValueError(f"channel_scale must hold {C} (per channel) or {B * C} (per item and channel) "
                              f"values, got shape {tuple(scale_t.shape)}")
+    handle = get_library_handle(dev)
+    L = _lib.load()
+    ptr = lambda t: 0 if t is None else t.data_ptr()  # noqa: E731
+    if host_chunks is None:
+        # one native call: stream, descriptors, scale, pair buffer and the
+        # beamforming itself (ffdas_das_call); beta is 0
+        od = out_t.shape
+        q = array("q", [handle.h.value, _raw_stream(dev.index), ptr(srcpos_t), ptr(srcdir_t), _bits(wavenum), ptr(xt),
+                        _FFDAS_DTYPE[xt.dtype], *_x_layout(xt, channels_trailing), ptr(dstpos_t), ptr(offsets_t),
+                        ptr(weights_t), idx_t.shape[0] if idx_t is not None else 0, ptr(idx_t), ptr(out_t),
+                        _FFDAS_DTYPE.get(out_t.dtype, DataType.R_32F), ctype, int(algorithm), ptr(scale_t),
+                        scale_t.numel() if scale_t is not None else 0, *(pair_buffer or (0, 0)), idx_t is not None,
+                        len(od), *od, *out_t.stride()])
+        _lib.check(L.ffdas_das_call(q.buffer_info()[0], len(q)))
+        if out is not None:
+            return out
+        return _from_torch_like(out_t, x)
+
+    handle.set_stream(_raw_stream(dev.index))
+    beta = _beta_buffer(out_t.dtype)
+    x_desc = _x_desc(xt, channels_trailing)
+    o_desc = _lib.TensorDesc(list(out_t.shape), list(out_t.stride()),
+                             _FFDAS_DTYPE.get(out_t.dtype, DataType.R_32F))
+    ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    if scale_t is not None:
         handle.set_channel_scale(scale_t.data_ptr(), scale_t.numel())
     try:
-        if host_chunks is not None:
-            code = L.ffdas_das_from_host(handle.h, ptr(srcpos_t), ptr(srcdir_t), float(wavenum), x_desc.desc,
-                                         ptr(xt), ptr(dstpos_t), ptr(offsets_t), ptr(weights_t),
-                                         ctypes.cast(beta, ctypes.c_void_p), o_desc.desc, ptr(out_t), int(ctype),
-                                         int(algorithm), int(host_chunks))
-        elif idx_t is None:
-            code = L.ffdas_das(handle.h, ptr(srcpos_t), ptr(srcdir_t), float(wavenum), x_desc.desc, ptr(xt),
-                               ptr(dstpos_t), ptr(offsets_t), ptr(weights_t), ctypes.cast(beta, ctypes.c_void_p),
-                               o_desc.desc, ptr(out_t), int(ctype), int(algorithm))
-        else:
-            code = L.ffdas_das_sparse(handle.h, ptr(srcpos_t), ptr(srcdir_t), float(wavenum), x_desc.desc,
-                                      ptr(xt), ptr(dstpos_t), ptr(offsets_t), ptr(weights_t), int(idx_t.shape[0]),
-                                      ptr(idx_t), ctypes.cast(beta, ctypes.c_void_p), o_desc.desc, ptr(out_t),
-                                      int(ctype), int(algorithm))
+        code = L.ffdas_das_from_host(handle.h, ptr(srcpos_t), ptr(srcdir_t), float(wavenum), x_desc.desc,
+                                     ptr(xt), ptr(dstpos_t), ptr(offsets_t), ptr(weights_t),
+                                     ctypes.cast(beta, ctypes.c_void_p), o_desc.desc, ptr(out_t), int(ctype),
+                                     int(algorithm), int(host_chunks))
     finally:
         if scale_t is not None:
             handle.set_channel_scale(None, 0)
@@ -360,7 +391,7 @@ def sparse_select(weights, k: int, offsets=None):
     sw = torch.empty((k, *spatial), dtype=torch.float32, device=dev)
     so = torch.empty((k, *spatial), dtype=torch.float32, device=dev) if o_t is not None else None
     handle = get_library_handle(dev)
-    handle.set_stream(torch.cuda.current_stream(dev).cuda_stream)
+    handle.set_stream(_raw_stream(dev.index))
     ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
     _lib.check(_lib.load().ffdas_sparse_select(handle.h, ptr(w_t), ptr(o_t), int(n), int(V), int(k), ptr(idx),
                                                ptr(sw), ptr(so)))

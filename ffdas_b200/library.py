@@ -29,11 +29,14 @@ def get_library_handle(device=None) -> _lib.Handle:
     if device is None:
         index = torch.cuda.current_device()
     else:
-        index = torch.device(device).index
+        index = (device if type(device) is torch.device else torch.device(device)).index
         if index is None:
             index = torch.cuda.current_device()
     if _lib.device_get() != index:
         _lib.device_set(index)
+    h = _handles.get(index)
+    if h is not None:
+        return h
     with _lock:
         h = _handles.get(index)
         if h is None:

@@ -14,7 +14,7 @@ import torch
 
 from . import _lib
 from ._lib import DataType
-from .das import _from_torch_like, _to_torch
+from .das import _from_torch_like, _raw_stream, _to_torch
 from .library import get_library_handle
 
 _DTYPES = {
@@ -72,7 +72,7 @@ def truncate_rank(x, start: int, stop: int | None = None, *, out=None):
     xd = _lib.TensorDesc((m, n), None, dt)
     od = _lib.TensorDesc((m, n), None, dt)
     handle = get_library_handle(dev)
-    handle.set_stream(torch.cuda.current_stream(dev).cuda_stream)
+    handle.set_stream(_raw_stream(dev.index))
     _lib.check(_lib.load().ffdas_truncate_rank(handle.h, xd.desc, xc.data_ptr(), int(start), int(stop), od.desc,
                                                target.data_ptr()))
     if ot is not None:

@@ -19,6 +19,7 @@
  *   - ffdas_get_last_kernel_info: which kernel the last call launched.
  *   - ffdas_set_pair_buffer / ffdas_das_pair_bytes: interpolation pairs kept
  *     from a forward call for the backward on the same data.
+ *   - ffdas_das_call / ffdas_das_backward_call: one call with packed arguments.
  *   - ffdas_set_channel_scale: per-channel gain applied at the ingest.
  *   - ffdas_das_static: forward without device allocation or handle.
  *   - ffdas_das_from_host: forward on host-resident channel data, uploads
@@ -330,6 +331,27 @@ FFDAS_API ffdas_error_t ffdas_das_backward(
 FFDAS_API ffdas_error_t ffdas_set_pair_buffer(ffdas_handle_t handle, void *buffer, size_t bytes);
 FFDAS_API ffdas_error_t ffdas_das_pair_bytes(ffdas_tensor_desc_t x_desc, ffdas_compute_type_t compute_type,
                                              size_t *bytes);
+
+/* New: one call for a binding whose per-argument cost counts (small frames are
+ * over on the GPU in a few microseconds): sets the handle's stream, builds both
+ * descriptors, applies a channel scale and a pair buffer for this call and runs
+ * ffdas_das / ffdas_das_sparse with beta 0.  q holds n int64 values (pointers
+ * as integers):
+ *   handle, stream, srcpos, srcdir, wavenum (bits of a double), x, x dtype,
+ *   x ndim (3 or 4), four x dims, four x strides, dstpos, offsets, weights,
+ *   sparse_count, sparse_indices, out, out dtype, compute type, algorithm,
+ *   channel scale, its count, pair buffer, its bytes, sparse (0 / 1),
+ *   out ndim, out dims, out strides.
+ * A scale or pair buffer of 0 leaves the handle's own setting; one given is
+ * cleared after the call. */
+FFDAS_API ffdas_error_t ffdas_das_call(const int64_t *q, int64_t n);
+
+/* New: the same for ffdas_das_backward:
+ *   handle, stream, srcpos, srcdir, wavenum, x, x dtype, x ndim, four dims, four
+ *   strides, dstpos, offsets, weights, sparse_count, sparse_indices, grad_out,
+ *   its dtype, grad_x, grad_offsets, grad_weights, grad_dstpos, grad_srcpos,
+ *   pair buffer, its bytes, grad_out ndim, dims, strides. */
+FFDAS_API ffdas_error_t ffdas_das_backward_call(const int64_t *q, int64_t n);
 
 /* New: ffdas_das on channel data in host memory (page-locked for the copies
  * to overlap; pageable memory works, serially).  Same arguments as ffdas_das
