@@ -567,6 +567,33 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         return launch_iq(h, pb, xd.dtype, kind, a.x, gain, gain_bstride, gp, IW.get<void>());
     }
 
+    // ---- das_sparse without a schedule: a lane per list entry on staged sample
+    // windows (das_entries.cuh) where the lists are long enough; the gather
+    // kernel else.  (A pair buffer stays unfilled: its adjoint reads no pairs.)
+    if (!h.has_config && od.dtype == FFDAS_R_32F && entries_supported(pb, kind)) {
+        const float *gain = nullptr;
+        int gain_bstride = 0;
+        FFDAS_TRY(channel_gain(h, pb, &gain, &gain_bstride));
+        workspace EW(h);
+        FFDAS_TRY(EW.alloc(entries_workspace(pb)));
+        gather_params gp;
+        std::memset(&gp, 0, sizeof(gp));
+        gp.C = pb.C; gp.S = pb.S; gp.n_events = pb.n_events; gp.B = pb.B; gp.V = pb.V;
+        gp.D0 = pb.D0; gp.D1 = pb.D1; gp.D2 = pb.D2;
+        gp.srcpos = a.srcpos; gp.srcdir = reinterpret_cast<const float4 *>(a.srcdir);
+        gp.dstpos = a.dstpos; gp.offsets = a.offsets; gp.weights = a.weights;
+        gp.sparse_idx = a.sparse_indices;
+        gp.out = a.out;
+        gp.out_bstride = pb.out_bstride;
+        read_beta(od.dtype, a.beta, gp.beta_re, gp.beta_im, gp.beta_zero);
+        h.last = ffdas_kernel_info_t{};
+        h.last.storage = kind;
+        h.mark_start();
+        const ffdas_error_t err = launch_entries(h, pb, xd.dtype, kind, a.x, gain, gain_bstride, gp, EW.get<void>());
+        h.mark_stop();
+        return err;
+    }
+
     // ---- ingest: x -> pair rows (workspace) ----
     const int64_t npad = pair_row_length(pb.N);
     const int64_t rows = (int64_t)pb.B * pb.C * pb.S;

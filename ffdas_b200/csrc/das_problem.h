@@ -132,6 +132,14 @@ ffdas_error_t launch_staged_bwd(ffdas_context &h, const das_problem &pb, int kin
 bool mma_supported(const das_problem &pb, ffdas_datatype_t xt, ffdas_datatype_t ot, int kind);
 ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call &a, float *out);
 
+// das_sparse on sorted list entries (csrc/das_entries.cuh): real storage kinds,
+// f32 output, lists of at most 64 entries over at most 480 events; no pair
+// rows.  ws is entries_workspace() bytes; gain as in the ingest.
+bool entries_supported(const das_problem &pb, int kind);
+size_t entries_workspace(const das_problem &pb);
+ffdas_error_t launch_entries(ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt, int kind, const void *x,
+                             const float *gain, int gain_bstride, gather_params gp, void *ws);
+
 // das_sparse as one persistent launch over (tile, channel slice) work items,
 // longest tiles first (csrc/das_sparse_items.cuh): real pair storage, f32
 // output, lists of at most 64 entries.  gp holds 256-voxel tiles and the

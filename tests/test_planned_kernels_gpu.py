@@ -124,6 +124,86 @@ def test_iq_adjoint(B, S, C, N, pitch):
         assert oracle.rel_l2(a.grad.cpu().numpy(), b.grad.numpy()) < tol, name
 
 
+def _lists(S, n, V, seed, dup=False):
+    g = torch.Generator().manual_seed(seed)
+    idx = torch.argsort(torch.rand((S, *V), generator=g), dim=0)[:n].int()
+    if dup:
+        idx[-1] = idx[0]
+    idx[0, 0, 0] = S + 3                     # an event outside x adds nothing
+    idx[1 % n, 1, 1] = -1
+    w = torch.rand((n, *V), generator=g) + 0.1
+    w[torch.rand((n, *V), generator=g) < 0.3] = 0.0
+    return idx.contiguous(), w
+
+
+def _gather_kernel(*args, **kw):
+    h = ffdas_b200.get_library_handle(torch.device(DEV))
+    h.set_config({"variant": 1})
+    try:
+        return ffdas_b200.das_sparse(*args, **kw)
+    finally:
+        h.set_config(None)
+
+
+def _against_gather(x, src, dst, offs, w, idx, srcdir=None):
+    """Both kernels on the whole grid, the oracle on every 13th and 7th pixel: (got, oracle's pixels)."""
+    args = _dev(x, src, dst, offs, w, idx)
+    kw = {} if srcdir is None else {"srcdir": srcdir.to(DEV)}
+    got = ffdas_b200.das_sparse(*args, **kw)
+    assert _info()["variant"] == 9
+    ref = _gather_kernel(*args, **kw)
+    assert _info()["variant"] == 1
+    cut = (slice(None), slice(None, None, 13), slice(None, None, 7))
+    few = _oracle(x, src, dst[cut[1:]].contiguous(), offs[cut].contiguous(), w[cut].contiguous(),
+                  sparse_indices=idx[cut].contiguous(), srcdir=srcdir)
+    return got.cpu().numpy(), ref.cpu().numpy(), few
+
+
+# (2^27 list places and more; items and channels off the box sizes, lists of
+# every event and of a few, rows that are copied and rows read in place)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.int16])
+@pytest.mark.parametrize("B,C,S,n,N,pitch", [(4, 1000, 4, 4, 512, (1.0, 0.5)), (3, 1101, 6, 5, 509, (4.0, 0.5)), (2, 400, 20, 20, 512, (0.3, 0.3)),
+                                             (1, 490, 64, 32, 384, (1.5, 0.5)), (5, 1100, 3, 3, 128, (0.5, 0.5)),
+                                             (1, 327, 180, 48, 128, (0.7, 0.4))], ids=str)
+def test_sorted_entries(dtype, B, C, S, n, N, pitch):
+    x, src, dst, offs, _ = _problem(B, C, S, N, 131, 67, pitch, seed=n, n=n)
+    x = (x * 300).round().to(dtype) if dtype == torch.int16 else x.to(dtype)
+    idx, w = _lists(S, n, (131, 67), seed=S, dup=True)
+    got, ref, few = _against_gather(x, src, dst, offs, w, idx, _cone(C) if n % 2 else None)
+    assert oracle.rel_l2(got, ref) < TOL
+    assert oracle.rel_l2(got[:, ::13, ::7], few) < TOL
+
+
+def test_sorted_entries_strided_data():
+    # channels trailing, a row pitch of its own, and an offset that is not 16-byte aligned
+    x, src, dst, offs, _ = _problem(2, 500, 16, 300, 131, 67, n=16)
+    idx, w = _lists(16, 16, (131, 67), seed=3)
+    args = _dev(src, dst, offs, w, idx)
+    ref = ffdas_b200.das_sparse(x.to(DEV), *args)
+    assert _info()["variant"] == 9
+    wide = torch.zeros((2, 500, 16, 330), device=DEV)
+    for first in (0, 8, 3):
+        wide[..., first:first + 300] = x.to(DEV)
+        got = ffdas_b200.das_sparse(wide[..., first:first + 300], *args)   # sums in another order at most
+        assert torch.linalg.norm(got - ref) < 1e-6 * torch.linalg.norm(ref)
+    xt = x.transpose(1, 2).contiguous().to(DEV)
+    got = ffdas_b200.das_sparse(xt, *args, channels_trailing=True)
+    assert torch.linalg.norm(got - ref) < 1e-6 * torch.linalg.norm(ref)
+
+
+def test_sorted_entries_non_finite_delay_stays_in_its_voxel():
+    x, src, dst, offs, _ = _problem(4, 1000, 4, 512, 131, 67, n=4)
+    idx, w = _lists(4, 4, (131, 67), seed=2)
+    w[2, 10, 10], idx[2, 10, 10] = 1.0, 1
+    offs[2, 10, 10] = float("nan")
+    dst[40, 20, 0] = float("inf")
+    got, ref, _ = _against_gather(x, src, dst, offs, w, idx)
+    ok = np.ones((131, 67), bool)
+    ok[10, 10] = ok[40, 20] = False
+    assert np.isnan(got[:, 10, 10]).all() and (np.isfinite(got[:, 40, 20]) == np.isfinite(ref[:, 40, 20])).all()
+    assert oracle.rel_l2(got[:, ok], ref[:, ok]) < TOL
+
+
 @pytest.mark.parametrize("B,C,S,N,pitch", [(32, 9, 1, 256, (1.0, 0.5)), (33, 40, 3, 250, (1.5, 0.5)), (64, 17, 4, 504, (6.0, 0.5)),
                                            (270, 8, 2, 160, (0.5, 0.5))], ids=str)
 def test_tensor_core_batches(B, C, S, N, pitch):
