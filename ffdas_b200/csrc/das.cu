@@ -525,7 +525,8 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         const bool asked = h.has_config && h.config.variant == 5;
         const bool planner = !h.has_config || h.config.variant == 0;
         const int64_t units = pb.V * pb.C * (int64_t)pb.S * pb.B;
-        if (asked || (planner && units <= (pb.B == 1 ? kDirectUnits : kDirectUnitsBatched))) {
+        if (asked || (planner && units <= (pb.B == 1 ? kDirectUnits : kDirectUnitsBatched) &&
+                      !(!h.has_config && pb.B == 1 && pb.V >= kDirectFrameVoxels && units >= kDirectFrameUnits))) {
             double br = 0.0, bi = 0.0;
             int bz = 1;
             read_beta(od.dtype, a.beta, br, bi, bz);

@@ -4,10 +4,17 @@
 // 128 channels) is over in microseconds, so the cost of a call is its launch
 // chain: the pair ingest, the staged kernel's pipeline fill and the handful
 // of windows each CTA stages.  This kernel is the whole call in one launch
-// and no workspace: `split` consecutive lanes share a voxel and take every
-// split-th channel, read x[k] and x[k+1] where the tap lands (L1/L2 gathers;
-// the channel data of such a frame is a megabyte or two), and add their
-// partial sums with warp shuffles.
+// and no workspace: `split` threads share a voxel and take every split-th
+// channel, read x[k] and x[k+1] where the tap lands (L1/L2 gathers; the channel
+// data of such a frame is a megabyte or two), and add their partial sums.
+//
+// The threads of a voxel lie in different warps (up to 8, their sums meet in
+// shared memory) before they lie in different lanes: the lanes of a warp are
+// then neighbouring voxels on ONE channel row, whose taps fall into a few cache
+// lines.  Lanes on different channels read up to 32 lines per load, and the
+// rate of those set the time (kernel, lanes first and warps first: 120 channels,
+// 9 events, 9860 pixels 54 and 22 us; 84, 5, 24396: 37 and 31; 172, 1, 40248,
+// where few threads share a voxel: 21 in both).
 //
 // Arithmetic per (voxel, channel, event) is the reference's
 // (src/das/das_alg1_kernels.cuh:60-99, lerp = fma(t, x1 - x0, x0)): the same
@@ -50,6 +57,7 @@ constexpr int kDirectUnroll = 4;
 template <typename Tin, int BT>
 __global__ void __launch_bounds__(kDirectThreads) das_direct_kernel(const direct_params p) {
     extern __shared__ float4 chan[];   // (x, y, z, 0) per channel
+    __shared__ float red[BT][kDirectThreads / 32][32];
     const int C = p.C, S = p.S, split = p.split;
     const int64_t V = p.V;
     if (p.chan_smem) {
@@ -57,9 +65,10 @@ __global__ void __launch_bounds__(kDirectThreads) das_direct_kernel(const direct
             chan[i] = make_float4(__ldg(p.srcpos + 3 * i), __ldg(p.srcpos + 3 * i + 1), __ldg(p.srcpos + 3 * i + 2), 0.f);
         __syncthreads();
     }
-    const int64_t gt = (int64_t)blockIdx.x * kDirectThreads + threadIdx.x;
-    const int64_t v = gt >> p.split_log2;
-    const int part = (int)(gt & (split - 1));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wl = min(p.split_log2, 3), ll = p.split_log2 - wl;   // warps and lanes of a voxel (log2)
+    const int warp_part = warp & ((1 << wl) - 1), part = (warp_part << ll) | (lane & ((1 << ll) - 1));
+    const int64_t v = (int64_t)blockIdx.x * (kDirectThreads >> p.split_log2) + ((warp >> wl) << (5 - ll)) + (lane >> ll);
     const bool active = v < V;
     const int b0 = (int)blockIdx.y * BT;
     float acc[BT];
@@ -131,10 +140,21 @@ __global__ void __launch_bounds__(kDirectThreads) das_direct_kernel(const direct
         for (; c0 + (kDirectUnroll - 1) * split < C; c0 += stride) step(c0, std::false_type{});
         if (c0 < C) step(c0, std::true_type{});
     }
-    // partial sums of the voxel's split lanes (consecutive lanes of one warp)
-    for (int off = split >> 1; off > 0; off >>= 1) {
+    // partial sums: the voxel's lanes, then its warps in order
+    for (int off = 1 << ll >> 1; off > 0; off >>= 1) {
 #pragma unroll
         for (int bi = 0; bi < BT; bi++) acc[bi] += __shfl_xor_sync(0xffffffffu, acc[bi], off);
+    }
+    if (wl > 0) {
+#pragma unroll
+        for (int bi = 0; bi < BT; bi++) red[bi][warp][lane] = acc[bi];
+        __syncthreads();
+        if (warp_part == 0) {
+            for (int w = 1; w < (1 << wl); w++) {
+#pragma unroll
+                for (int bi = 0; bi < BT; bi++) acc[bi] += red[bi][warp + w][lane];
+            }
+        }
     }
     if (!active || part != 0) return;
 #pragma unroll
@@ -159,7 +179,7 @@ static ffdas_error_t launch_direct_t(ffdas_context &h, const direct_params &dp) 
     const int64_t bchunks = (dp.B + BT - 1) / BT;
     if (blocks > INT32_MAX || bchunks > 65535) return FFDAS_ERROR_DIMS_TOO_LARGE;
     const size_t smem = dp.chan_smem ? (size_t)dp.C * sizeof(float4) : 0;
-    if (smem > 48 * 1024) {   // the attribute belongs to the device: set it for each one
+    if (smem > 40 * 1024) {   // (with up to 4 KB of partial sums) the attribute belongs to the device: set it for each one
         static std::atomic<unsigned long long> done{0ull};
         int dev = 0;
         FFDAS_CUDA(cudaGetDevice(&dev));
@@ -225,7 +245,7 @@ ffdas_error_t launch_direct(ffdas_context &h, const das_problem &pb, ffdas_datat
     dp.bstride = (int)pb.x_bstride; dp.cstride = (int)pb.x_cstride; dp.sstride = (int)pb.x_sstride;
     dp.chan_smem = pb.C <= kDirectSmemChannels;
     dp.B = pb.B; dp.C = pb.C; dp.S = pb.S; dp.N = pb.N; dp.V = pb.V;
-    // lanes per voxel (power of two, at most 32 and at most the channel
+    // threads per voxel (power of two, at most 32 and at most the channel
     // count): the schedule's tile_x, else the most that keeps the launch
     // within two waves of resident threads (measured: the per-thread channel
     // loop is latency-bound, so more lanes pay until the second wave fills)
@@ -253,7 +273,7 @@ ffdas_error_t launch_direct(ffdas_context &h, const das_problem &pb, ffdas_datat
     dp.beta_zero = beta_zero;
     h.last = ffdas_kernel_info_t{};
     h.last.variant = 5;
-    h.last.tile_x = split;     // lanes per voxel
+    h.last.tile_x = split;     // threads per voxel
     h.last.tile_y = 1; h.last.tile_z = 1;
     h.last.batch_tile = BT >= 4 ? 4 : BT;
     h.last.event_chunk = 1;
