@@ -145,8 +145,8 @@ __device__ __forceinline__ void iq_produce(const staged_params &p, const CUtenso
             const float ez = fmaxf(fabsf(pz - ab[2]), fabsf(pz - ab[5]));
             const float rmin = sqrtf(dx * dx + dy * dy + dz * dz);
             const float rmax = sqrtf(ex * ex + ey * ey + ez * ez);
-            const float lo = floorf(sm.ofs_lo[j] + rmin) - 2.f;
-            const float hi = floorf(sm.ofs_hi[j] + rmax) + 2.f;
+            float lo, hi;
+            tap_range(sm.ofs_lo[j], sm.ofs_hi[j], rmin, rmax, lo, hi);
             // taps k of the record: 0 <= k < N - 1, each with its next sample
             if (lo == lo && hi == hi && hi >= 0.f && lo < (float)(p.N - 1)) {
                 k0 = (int)fmaxf(lo, 0.f) & ~(IG::align - 1);
@@ -556,13 +556,13 @@ __global__ void __launch_bounds__(kStThreads, 2) das_iq_bwd_kernel(const iq_para
                         for (int j = 0; j < SC; j++) {
                             const uint32_t rr = mb[j] - k0p[j];
                             const bool in_rec = mb[j] - kFloorMagicBits < nlast;
-                            const uint32_t at = rr < (uint32_t)(WB - 1) && in_rec
-                                                    ? groups + j * IG::group_bytes + rr * (uint32_t)IG::sample_bytes
-                                                    : zero_u32;
+                            const bool staged = rr < (uint32_t)(WB - 1) && in_rec;
+                            const uint32_t at = staged ? groups + j * IG::group_bytes + rr * (uint32_t)IG::sample_bytes
+                                                       : zero_u32;
                             const bool ovfw = !FAST && k0p[j] == kOvf;
                             // a tap outside the record scatters zeros (into its window's
                             // bins, or the zero-only bin past the window)
-                            const float ws = in_rec ? w[j] * fscale : 0.f;
+                            const float ws = staged ? w[j] * fscale : 0.f;
                             const float wst = ws * t[j];
                             const uint32_t gb = gwin_u32 + (j * BT * 2 * GS + min(rr, (uint32_t)WB)) * 4;
                             float qj = 0.f, qx = 0.f;
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(kStThreads, 2) das_iq_bwd_kernel(const iq_para
                                     red_shared_add_at<(b * 2 + 1) * GS * 4 + 4>(gb, by - (int)kFloorMagicBits);
                                 } else if constexpr (!FAST) {
                                     if (gx && in_rec && w[j] != 0.f && b0 + b < p.B) {
-                                        if (fixed && !ovfw && rr < (uint32_t)WB) {
+                                        if (fixed && !ovfw && rr < (uint32_t)(WB - 1)) {
                                             const int ax = fix_bits_fma(u.x, ws), bx = fix_bits_fma(u.x, wst);
                                             const int ay = fix_bits_fma(u.y, ws), by = fix_bits_fma(u.y, wst);
                                             red_shared_add_at<b * 2 * GS * 4>(gb, ax - bx);
@@ -639,7 +639,8 @@ __global__ void __launch_bounds__(kStThreads, 2) das_iq_bwd_kernel(const iq_para
                             const int grp = win / BT, b = win % BT;
                             const int cl = grp / SC, j = grp % SC;
                             kw = (int)(sm.meta[stage * kStWin + grp] - kFloorMagicBits);
-                            if (b0 + b >= p.B || c0 + cl >= cend) return nullptr;
+                            // (a window past the record, or read from the rows, has nothing in its bins)
+                            if (b0 + b >= p.B || c0 + cl >= cend || (unsigned)kw >= (unsigned)p.N) return nullptr;
                             return gx + (((int64_t)(b0 + b) * p.C + (c0 + cl)) * p.S + (e0 + j)) * p.N;
                         });
                     }

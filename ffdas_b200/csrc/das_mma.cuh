@@ -115,8 +115,8 @@ __device__ __forceinline__ mma_block mma_windows(const mma_params &p, const floa
     const float ez = fmaxf(fabsf(w.pz - box[2]), fabsf(w.pz - box[5]));
     // (a channel position that is not finite has no window: NaN, or nothing in
     // range; the builders spoil their voxels and the fix-up decides)
-    const float lo = floorf(olo + sqrtf(dx * dx + dy * dy + dz * dz)) - 2.f;
-    const float hi = floorf(ohi + sqrtf(ex * ex + ey * ey + ez * ez)) + 2.f;
+    float lo, hi;
+    tap_range(olo, ohi, sqrtf(dx * dx + dy * dy + dz * dz), sqrtf(ex * ex + ey * ey + ez * ez), lo, hi);
     if (!isfinite(w.px + w.py + w.pz) || !(hi >= 0.f) || !(lo < (float)(p.N - 1))) return w;
     w.k0 = (int)fmaxf(lo, 0.f) & ~7;
     w.len = (int)fminf(hi, (float)(p.N - 1)) - w.k0 + 1;

@@ -247,6 +247,23 @@ enum : int { kStageEmpty = 1, kStageFast = 2 };
 enum : int { kPassSkip = 1, kPassFast = 2 };
 constexpr float kSaneRange = 1048576.0f;   // 2^20: tau, offsets and distances below it keep |rounding| < 1 sample
 
+// [lo, hi] with lo + 1 <= floor(tau) <= hi - 1 for every tap of a tile: delays
+// olo .. ohi, distances rmin .. rmax.  A tap's distance rsq * rsqrt(rsq) is
+// within 2^-21 of its size of the true one, the bounds within 2^-22: less than
+// a sample up to 2^20.  Far delays that cancel far distances (a time origin
+// millions of samples away) meet the record all the same, and their windows
+// grow with that rounding; without it an in-record tap missed its window (left
+// out of the image, and in the adjoints added past its window's bins).
+__device__ __forceinline__ void tap_range(float olo, float ohi, float rmin, float rmax, float &lo, float &hi) {
+    lo = floorf(olo + rmin) - 2.f;
+    hi = floorf(ohi + rmax) + 2.f;
+    const float far = fmaxf(fabsf(olo), fabsf(ohi)) + rmax;
+    if (far > kSaneRange) {   // (no finite delay in the tile: lo = inf and hi = -inf stay)
+        if (lo <= 3e38f) lo -= 2e-6f * far;
+        if (hi >= -3e38f) hi += 2e-6f * far;
+    }
+}
+
 template <int WB, int K>
 constexpr size_t staged_smem_bytes() {
     // ring, one zero slot (the target of zero windows on the unclamped path), misc
@@ -823,8 +840,8 @@ __device__ __forceinline__ void staged_produce(const staged_params &p, const CUt
             const float ez = fmaxf(fabsf(pz - ab[2]), fabsf(pz - ab[5]));
             const float rmin = sqrtf(dx * dx + dy * dy + dz * dz);
             const float rmax = sqrtf(ex * ex + ey * ey + ez * ez);
-            const float lo = floorf(sm.ofs_lo[j] + rmin) - 2.f;
-            const float hi = floorf(sm.ofs_hi[j] + rmax) + 2.f;
+            float lo, hi;
+            tap_range(sm.ofs_lo[j], sm.ofs_hi[j], rmin, rmax, lo, hi);
             // Every tap's floor(tau) lies in [lo + 1, hi - 1] when the delays,
             // distances and tau stay below 2^20 in magnitude (rounding < 1 sample).
             const bool sane = fabsf(lo) <= kSaneRange && fabsf(hi) <= kSaneRange && rmax <= kSaneRange;
@@ -965,8 +982,8 @@ __device__ __forceinline__ void staged_produce_pass2(const staged_params &p, con
             const float n2 = dx * dx + dy * dy + dz * dz, x2 = ex * ex + ey * ey + ez * ez;
             const float rmin = n2 > 0.f ? n2 * rsqrtf(n2) : 0.f;
             const float rmax = x2 > 0.f ? x2 * rsqrtf(x2) : 0.f;
-            const float lo = floorf(olo + rmin) - 2.f;
-            const float hi = floorf(ohi + rmax) + 2.f;
+            float lo, hi;
+            tap_range(olo, ohi, rmin, rmax, lo, hi);
             // Every tap's floor(tau) lies in [lo + 1, hi - 1] when the delays,
             // distances and tau stay below 2^20 in magnitude (rounding < 1 sample).
             const bool sane = fabsf(lo) <= kSaneRange && fabsf(hi) <= kSaneRange && rmax <= kSaneRange;
@@ -1602,8 +1619,8 @@ __device__ __forceinline__ void staged_produce_batch(const staged_params &p, con
             const float ez = fmaxf(fabsf(pz - ab[2]), fabsf(pz - ab[5]));
             const float rmin = sqrtf(dx * dx + dy * dy + dz * dz);
             const float rmax = sqrtf(ex * ex + ey * ey + ez * ez);
-            const float lo = floorf(sm.ofs_lo[j] + rmin) - 2.f;
-            const float hi = floorf(sm.ofs_hi[j] + rmax) + 2.f;
+            float lo, hi;
+            tap_range(sm.ofs_lo[j], sm.ofs_hi[j], rmin, rmax, lo, hi);
             if (lo == lo && hi == hi && hi >= 0.f && lo < (float)p.npad) {
                 const int k0 = ((int)fmaxf(lo, -(float)WB)) & ~(staged_traits<K>::align_pairs - 1);
                 const int k1 = (int)fminf(hi, (float)p.npad + WB);
@@ -2024,7 +2041,7 @@ __global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_kernel(const sta
                         flush_bins<WB, kRegion>(gstage, cx.lane, cx.warp, finv, [&](int win, int &kw) -> float * {
                             const int cl = win / SC, j = win % SC;
                             kw = (int)(sm.meta[stage * kStWin + win] - kFloorMagicBits);
-                            if (c0 + cl >= cend) return nullptr;
+                            if (c0 + cl >= cend || kw >= p.N) return nullptr;
                             return p.gx + (((int64_t)cx.b * p.C + (c0 + cl)) * p.S + (e0 + j)) * p.N;
                         });
                     }
@@ -2397,7 +2414,7 @@ __global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_batch_kernel(con
                             const int grp = win / BT, bi = win % BT;
                             const int cl = grp / SC, j = grp % SC;
                             kw = (int)(sm.meta[stage * kStWin + grp] - kFloorMagicBits);
-                            if (b0 + bi >= p.B || c0 + cl >= cend) return nullptr;
+                            if (b0 + bi >= p.B || c0 + cl >= cend || kw >= p.N) return nullptr;
                             return p.gx + (((int64_t)(b0 + bi) * p.C + (c0 + cl)) * p.S + (e0 + j)) * p.N;
                         });
                     }

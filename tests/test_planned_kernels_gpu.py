@@ -77,6 +77,45 @@ def test_planned_tiles(pitch, B, S, cone):
     assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL
 
 
+def _with_config(config, f, *args, **kw):
+    h = ffdas_b200.get_library_handle(torch.device(DEV))
+    h.set_config(config)
+    try:
+        return f(*args, **kw)
+    finally:
+        h.set_config(None)
+
+
+@pytest.mark.parametrize("dtype,B,S,C", [(torch.float32, 1, 5, 1200), (torch.float32, 3, 4, 200), (torch.complex64, 1, 4, 33),
+                                         (torch.complex64, 3, 5, 20), (torch.float16, 32, 3, 33)], ids=str)
+@pytest.mark.parametrize("far", [2.0 ** 22, 2.0 ** 28])
+def test_far_delays_that_cancel_far_distances(dtype, B, S, C, far):
+    # distances round to 0.5 and to 32 samples: every kernel takes the same taps as
+    # the gather kernels, which test each one by itself (TOL: the same FP32 taps
+    # summed in another order, weights of 22 bits in the products)
+    x, src, dst, offs, w = _problem(B, C, S, 500, 131, 67, dtype=dtype)
+    dst[..., 2] += far
+    offs = offs - far + 100.0
+    cplx = dtype.is_complex
+    args = _dev(x, src, dst, offs, w)
+    got = ffdas_b200.das(*args)
+    assert _info()["variant"] == (10 if dtype == torch.float16 else 2)
+    ref = _with_config({"variant": 1}, ffdas_b200.das, *args)
+    assert _info()["variant"] == 1 and ref.abs().max() > 0
+    assert oracle.rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < TOL
+    if dtype == torch.float16:
+        return
+    gy = torch.randn(got.shape, generator=torch.Generator().manual_seed(1), dtype=got.dtype).to(DEV)
+    grads = []
+    for config in (None, {"variant": 3}):
+        leaf = [t.clone().requires_grad_(True) for t in args]
+        _with_config(config, lambda: ffdas_b200.das(*leaf).backward(gy))
+        assert _info()["variant"] == (8 if cplx else 3 if config else 4)
+        grads.append([t.grad.cpu().numpy() for t in leaf])
+    for a, b in zip(*grads):
+        assert oracle.rel_l2(a, b) < TOL
+
+
 @pytest.mark.parametrize("dtype", [torch.complex64, torch.complex32])
 @pytest.mark.parametrize("B,S,C,N", [(1, 1, 24, 500), (1, 4, 17, 40), (2, 5, 33, 501), (3, 3, 9, 502), (4, 2, 30, 96), (5, 8, 40, 500)])
 @pytest.mark.parametrize("pitch", [(0.7, 0.5), (6.0, 0.5)], ids=str)

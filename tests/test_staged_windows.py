@@ -208,3 +208,62 @@ def test_fast_path_windows_cover_taps_smaller_volume(WB):
 def test_fast_path_plane_wave_frame():
     wl = W.plane2d(scale=0.5)
     check_fast(wl, 64, T0=512, T1=1, SC=1, max_tiles=16)
+
+
+# ---------------------------------------------------------------------------
+# Far distances cancelled by far delays (tap_range in csrc/das_staged.cuh)
+
+F = np.float32
+
+
+def tap_range(olo, ohi, rmin, rmax, grow=True):
+    lo = np.floor(F(olo + rmin)) - F(2)
+    hi = np.floor(F(ohi + rmax)) + F(2)
+    far = F(max(abs(olo), abs(ohi)) + rmax)
+    if grow and far > SANE:
+        lo, hi = F(lo - F(2e-6) * far), F(hi + F(2e-6) * far)
+    return lo, hi
+
+
+def far_tile(far, seed=0):
+    """A 16 x 16 tile about `far` wavelengths away, 33 channels, delays that bring its taps into a 500-sample record."""
+    rng = np.random.default_rng(seed)
+    p = np.zeros((256, 3), F)
+    p[:, 2] = F(far) + np.repeat(np.arange(16), 16).astype(F)
+    p[:, 0] = np.tile(np.arange(16), 16)
+    src = np.zeros((33, 3), F)
+    src[:, 0] = rng.uniform(-1, 1, 33) * (16 if far < 1e4 else 3000)
+    offs = (F(-far) + rng.uniform(100, 400, 256).astype(F)).astype(F)
+    return p, src, offs
+
+
+def missed_taps(far, grow):
+    p, src, offs = far_tile(far)
+    lo, hi = p.min(0), p.max(0)
+    missed = inside = 0
+    for c in src:
+        d = (p - c).astype(F)
+        rsq = ((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]).astype(F) + d[:, 2] * d[:, 2]).astype(F)
+        # rsqrtf errs by up to 2 units in the last place: both ends of it
+        rinv = (1 / np.sqrt(rsq.astype(np.float64))).astype(F)
+        gap = np.maximum(np.maximum(lo - c, c - hi), 0).astype(F)
+        ext = np.maximum(np.abs(c - lo), np.abs(c - hi)).astype(F)
+        rmin, rmax = F(np.sqrt((gap * gap).sum(dtype=F))), F(np.sqrt((ext * ext).sum(dtype=F)))
+        wlo, whi = tap_range(offs.min(), offs.max(), rmin, rmax, grow)
+        for ulp in (-2, 0, 2):
+            r = rsq.astype(np.float64) * (rinv.view(np.int32) + np.int32(ulp)).view(F).astype(np.float64)
+            k = np.floor((r + offs).astype(F))             # one rounding: fma(rsq, rinv, offset)
+            rec = (k >= 0) & (k < 499)
+            inside += rec.sum()
+            missed += (rec & ~((k >= wlo + 1) & (k <= whi - 1))).sum()
+    return missed, inside
+
+
+@pytest.mark.parametrize("far", [40.0, 4096.0, 2.0 ** 19, 2.0 ** 22, 2.0 ** 25, 2.0 ** 28])
+def test_tap_range_holds_far_taps(far):
+    missed, inside = missed_taps(far, True)
+    assert inside > 1000 and missed == 0
+
+
+def test_far_taps_miss_a_range_of_two_samples_margin():
+    assert missed_taps(2.0 ** 28, False)[0] > 0
