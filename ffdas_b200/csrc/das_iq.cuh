@@ -196,6 +196,14 @@ __device__ __forceinline__ void iq_event_phases(const iq_params &q, bool active,
         E[j] = (active && j < sc) ? iq_phase(ofs[j], q.turn_hi, q.turn_lo) : make_float2(0.f, 0.f);
 }
 
+// apply_directivity; an excluded channel has no factor either: one whose
+// position is not finite (its distance and factor are NaN) is excluded too, and
+// adds nothing.
+__device__ __forceinline__ void iq_directivity(recv_geom &g, float2 &R, const staged_ctx &cx, float4 c, float4 dir) {
+    apply_directivity(g, cx.vx, cx.vy, cx.vz, c.x, c.y, c.z, dir);
+    if (g.rsq == 1e30f) R = make_float2(0.f, 0.f);
+}
+
 // Floor split of the delays of two events of a channel (SC >= 2), or one.
 template <int SC>
 __device__ __forceinline__ void iq_split(const recv_geom &g, const float (&ofs)[SC], float (&t)[SC],
@@ -278,10 +286,8 @@ __global__ void __launch_bounds__(kStThreads, 3) das_iq_kernel(const iq_params q
                         const int c = c0 + cl;
                         const float4 cp = sm.chan_pos[stage * kStWin + cl];
                         recv_geom g = receive_geometry(cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z);
-                        const float2 R = iq_phase(g.rsq * g.rinv, q.turn_hi, q.turn_lo);
-                        if (p.srcdir)
-                            apply_directivity(g, cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z,
-                                              sm.chan_dir[stage * kStWin + cl]);
+                        float2 R = iq_phase(g.rsq * g.rinv, q.turn_hi, q.turn_lo);
+                        if (p.srcdir) iq_directivity(g, R, cx, cp, sm.chan_dir[stage * kStWin + cl]);
                         uint32_t k0p[SC], mb[SC];
                         float t[SC];
                         load_meta<SC>(sm.meta, stage, cl, k0p);
@@ -537,10 +543,8 @@ __global__ void __launch_bounds__(kStThreads, 2) das_iq_bwd_kernel(const iq_para
                         const int c = c0 + cl;
                         const float4 cp = sm.chan_pos[stage * kStWin + cl];
                         recv_geom gm = receive_geometry(cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z);
-                        const float2 R = iq_phase(gm.rsq * gm.rinv, qp.turn_hi, qp.turn_lo);
-                        if (p.srcdir)
-                            apply_directivity(gm, cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z,
-                                              sm.chan_dir[stage * kStWin + cl]);
+                        float2 R = iq_phase(gm.rsq * gm.rinv, qp.turn_hi, qp.turn_lo);
+                        if (p.srcdir) iq_directivity(gm, R, cx, cp, sm.chan_dir[stage * kStWin + cl]);
                         float2 h[BT];
 #pragma unroll
                         for (int b = 0; b < BT; b++)

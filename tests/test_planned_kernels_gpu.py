@@ -130,6 +130,19 @@ def test_iq_batch_tiles(dtype, B, S, C, N, pitch):
     assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL * (1 + abs(wn))
 
 
+def test_iq_excluded_channel_with_a_position_that_is_not_finite():
+    # outside every cone, as in the oracle: no tap of it, and no NaN from its phase
+    x, src, dst, offs, w = _problem(2, 12, 4, 300, 50, 37, dtype=torch.complex64)
+    src[5, 0], src[7, 2], dst[20, 10, 1] = float("nan"), float("inf"), float("nan")
+    leaf = [t.to(DEV).requires_grad_(i in (0, 3, 4)) for i, t in enumerate((x, src, dst, offs, w))]
+    got = ffdas_b200.das(*leaf, srcdir=_cone(12).to(DEV), wavenum=0.3)
+    assert _info()["variant"] == 2
+    ref = _oracle(x, src, dst, offs, w, srcdir=_cone(12), wavenum=0.3)
+    assert np.isfinite(ref).all() and oracle.rel_l2(got.detach().cpu().numpy(), ref) < TOL
+    got.backward(torch.ones_like(got))
+    assert all(torch.isfinite(leaf[i].grad).all() for i in (0, 3, 4))
+
+
 def test_iq_strided_data():
     # channels trailing, a row pitch of its own, and starts that are not 16-byte aligned
     x, src, dst, offs, w = _problem(3, 20, 4, 300, 50, 37, dtype=torch.complex64)
