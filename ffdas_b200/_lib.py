@@ -149,6 +149,7 @@ SIGNATURES = {
     "ffdas_measure_fp32_peak": (c_err, [c_handle, ctypes.POINTER(ctypes.c_double)]),
     "ffdas_get_device_status": (c_err, [c_handle, ctypes.POINTER(ctypes.c_int)]),
     "ffdas_debug_staged_drop_stage": (None, [ctypes.c_int]),
+    "ffdas_debug_no_tensor_maps": (None, [ctypes.c_int]),
 }
 
 _lib = None

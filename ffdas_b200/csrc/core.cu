@@ -32,6 +32,16 @@ int ffdas_take_debug_drop_stage() {
     return g_drop_stage.exchange(0);
 }
 
+static std::atomic<bool> g_no_tensor_maps{false};
+
+extern "C" FFDAS_API void ffdas_debug_no_tensor_maps(int enable) {
+    g_no_tensor_maps.store(enable != 0);
+}
+
+bool ffdas_debug_tensor_maps_off() {
+    return g_no_tensor_maps.load(std::memory_order_relaxed);
+}
+
 cudaError_t ffdas_raise_smem_limit(const void *func, int device, size_t bytes) {
     static std::mutex mu;
     static std::map<std::pair<const void *, int>, size_t> raised;

@@ -42,6 +42,11 @@ extern "C" FFDAS_API void ffdas_debug_fail_alloc_after(int n);
 extern "C" FFDAS_API void ffdas_debug_staged_drop_stage(int enable);
 int ffdas_take_debug_drop_stage();
 
+// Test hook: while set, the driver's tensor-map encoder counts as missing, so
+// calls take the kernels that do without TMA boxes.
+extern "C" FFDAS_API void ffdas_debug_no_tensor_maps(int enable);
+bool ffdas_debug_tensor_maps_off();
+
 struct ffdas_context {
     int device_id = 0;
     int arch_code = 0;

@@ -613,7 +613,10 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     // the geometry (das_tile_plan.cuh)
     const bool staged_ok = staged_supported(pb, kind) && od.dtype == FFDAS_R_32F;
     schedule s = plan_schedule(h, pb, kind, staged_ok);
-    const int plan_tile = s.variant == 2 && !h.has_config ? s.T0 * s.T1 * s.T2 : 0;
+    // (batch tiles and the 512-voxel tiles of one item read a plan; the 256-voxel
+    // kernel of a batch that cannot have TMA boxes does not)
+    const bool planned = s.variant == 2 && !h.has_config && (s.BT > 1 || s.T0 * s.T1 * s.T2 == 512);
+    const int plan_tile = planned ? s.T0 * s.T1 * s.T2 : 0;
     const int64_t plan_tiles = plan_tile && pb.C > 0 ? plan_max_tiles(pb, plan_tile) : 0;
     void *const plan = plan_tiles > 0 && plan_tiles <= INT32_MAX ? static_cast<char *>(Pbase) + pair_bytes + 64 : nullptr;
     if (plan) {

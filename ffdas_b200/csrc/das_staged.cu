@@ -36,7 +36,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
             fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
         cudaGetLastError();
     });
-    return fn;
+    return ffdas_debug_tensor_maps_off() ? nullptr : fn;
 }
 
 bool staged_supported(const das_problem &pb, int kind) {
@@ -274,6 +274,8 @@ ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, c
                                                      (float)gp.beta_re, gp.beta_zero, nullptr);
         FFDAS_TRY(ffdas_launch_check(h.stream));
     }
+    // (the 256-voxel kernel of one item reads no plan: it would run for both widths)
+    if (gp.plan && BT == 1 && gp.T0 * gp.T1 * gp.T2 != 2 * kStConsumers) return FFDAS_ERROR_INTERNAL;
     if (!gp.plan || BT > 1) return launch_staged_width(h, pb, kind, gp, SC, BT > 1 && gp.plan ? 64 : WB, BT, copy, grid);
     FFDAS_TRY(launch_staged_width(h, pb, kind, gp, SC, 32, BT, copy, grid));
     return launch_staged_width(h, pb, kind, gp, SC, 64, BT, copy, grid);

@@ -11,11 +11,14 @@ rounded across a sample boundary takes the neighbouring slope: with |d tau| up
 to 6e-5 a share 2 |d tau| of the taps does, each off by about 1.6 of its own size,
 so delay and position gradients are held to sqrt(1.2e-4) * 1.6 = 1.8e-2, to 2.5e-2.
 """
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 import ffdas_b200
+from ffdas_b200 import _lib
 from oracle import oracle
 from torch_ref import das_ref
 
@@ -75,6 +78,36 @@ def test_planned_tiles(pitch, B, S, cone):
     assert _info()["variant"] == 2
     ref = rep * _oracle(x, src, dst, offs, w, srcdir=_cone(41) if cone else None)
     assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL
+
+
+@pytest.mark.parametrize("B", [1, 3])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_calls_without_tensor_maps(B, beta):
+    # batches then run the 256-voxel kernel one item at a time, which reads no
+    # plan: once, in one width, channel slices and all
+    # (40 channels, repeated for one item to pass the direct kernel's range: an array of
+    # a thousand would lengthen its delays, and their rounding, beyond TOL's N = 600)
+    rep = 25 if B == 1 else 4
+    x, src, dst, offs, w = _problem(B, 40, 4, 600, 131, 67, (1.7, 0.5))
+    ref = rep * _oracle(x, src, dst, offs, w)
+    x, src = x.repeat(1, rep, 1, 1), src.repeat(rep, 1)
+    old = torch.randn(ref.shape, generator=torch.Generator().manual_seed(2))
+    args = _dev(x, src, dst, offs, w)
+    L, h, out = _lib.load(), ffdas_b200.get_library_handle(torch.device(DEV)), old.to(DEV)
+    b = ctypes.c_float(beta)
+    L.ffdas_debug_no_tensor_maps(1)
+    try:
+        h.set_stream(torch.cuda.current_stream().cuda_stream)
+        xd = _lib.TensorDesc(list(x.shape), None, _lib.DataType.R_32F)
+        od = _lib.TensorDesc(list(out.shape), None, _lib.DataType.R_32F)
+        p = [t.data_ptr() for t in args]
+        _lib.check(L.ffdas_das(h.h, p[1], None, 0.0, xd.desc, p[0], p[2], p[3], p[4],
+                               ctypes.cast(ctypes.byref(b), ctypes.c_void_p), od.desc, out.data_ptr(), 0, 0))
+        info = _info()
+    finally:
+        L.ffdas_debug_no_tensor_maps(0)
+    assert info["variant"] == 2 and info["copy_engine"] == 2 and info["batch_tile"] == 1
+    assert oracle.rel_l2(out.cpu().numpy(), ref + beta * old.numpy()) < TOL
 
 
 def _with_config(config, f, *args, **kw):
