@@ -121,6 +121,7 @@ SIGNATURES = {
     "ffdas_das_backward": (c_err, [c_handle, c_ptr, c_ptr, ctypes.c_float, c_desc, c_ptr, c_ptr, c_ptr, c_ptr,
                                    ctypes.c_int, c_ptr, c_desc, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
     "ffdas_das_call": (c_err, [ctypes.c_size_t, ctypes.c_int64]),
+    "ffdas_das_call_pair_bytes": (c_err, [ctypes.c_size_t, ctypes.c_int64, ctypes.POINTER(ctypes.c_size_t)]),
     "ffdas_das_backward_call": (c_err, [ctypes.c_size_t, ctypes.c_int64]),
     "ffdas_sparse_select": (c_err, [c_handle, c_ptr, c_ptr, ctypes.c_int, ctypes.c_int64, ctypes.c_int, c_ptr,
                                     c_ptr, c_ptr]),

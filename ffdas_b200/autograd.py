@@ -18,8 +18,7 @@ import torch
 
 from . import _lib
 from ._lib import DataType
-from .das import (_FFDAS_DTYPE, _astype, _bits, _check_spatial, _compute_type, _raw_stream, _run, _to_torch, _x_desc,
-                  _x_layout)
+from .das import _FFDAS_DTYPE, _astype, _bits, _check_spatial, _raw_stream, _run, _to_torch, _x_layout
 from .library import get_library_handle
 
 
@@ -33,20 +32,15 @@ class DASFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, srcpos, dstpos, offsets, weights, sparse_indices, opts: dict):
         ctx.opts = opts
-        ctx.pairs = None
         xt = x.detach()
-        # The forward builds its interpolation-pair rows into a buffer kept for
-        # the backward (ffdas_set_pair_buffer), which then skips building them
-        # again; only where the backward can run.
-        pair_buffer = None
-        if _backward_supported(xt, opts["wavenum"]):
-            nbytes = _lib.pair_bytes(_x_desc(xt, opts["channels_trailing"]), _compute_type(xt, False, False))
-            ctx.pairs = torch.empty(nbytes, dtype=torch.uint8, device=xt.device)
-            pair_buffer = (ctx.pairs.data_ptr(), nbytes)
+        # Where the forward builds interpolation-pair rows and the backward can run,
+        # they are kept in a buffer and the backward skips building them again.
+        keep = _backward_supported(xt, opts["wavenum"])
         out = _run(xt, srcpos.detach(), dstpos.detach(), offsets.detach(), weights.detach(), sparse_indices,
                    srcdir=opts["srcdir"], wavenum=opts["wavenum"], algorithm=0, use_fp16=opts["use_fp16"],
                    use_bf16=opts["use_bf16"], channels_trailing=opts["channels_trailing"], out=None,
-                   pair_buffer=pair_buffer)
+                   keep_pairs=keep)
+        out, ctx.pairs = out if keep else (out, None)
         ctx.save_for_backward(x, srcpos, dstpos, offsets, weights,
                               sparse_indices if sparse_indices is not None else torch.empty(0))
         ctx.has_sparse = sparse_indices is not None

@@ -460,6 +460,53 @@ static void read_beta(ffdas_datatype_t ot, const void *beta, double &re, double 
     zero = (re == 0.0 && im == 0.0) ? 1 : 0;
 }
 
+// The kernels a forward call takes: the small-problem kernel, the tensor cores,
+// the IQ batch tiles or the sorted list entries, which read x itself, or those
+// on pair rows.  keep_pairs: the caller set a pair buffer to fill.
+enum class route { direct, mma, iq, entries, pairs };
+
+static route forward_route(const ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt, ffdas_datatype_t ot,
+                           int kind, bool scaled, bool keep_pairs, bool beta_zero) {
+    // small problems: the whole call as one launch (not with a channel scale,
+    // which the ingest applies)
+    if (!scaled && direct_supported(pb, xt, ot, kind)) {
+        const bool asked = h.has_config && h.config.variant == 5;
+        const bool planner = !h.has_config || h.config.variant == 0;
+        const int64_t units = pb.V * pb.C * (int64_t)pb.S * pb.B;
+        if (asked || (planner && units <= (pb.B == 1 ? kDirectUnits : kDirectUnitsBatched) &&
+                      !(!h.has_config && pb.B == 1 && pb.V >= kDirectFrameVoxels && units >= kDirectFrameUnits)))
+            return route::direct;
+    }
+    if (h.has_config) return route::pairs;
+    // large half-precision batches (not with a pair buffer to fill, a channel
+    // scale or a prior image to keep)
+    if (!scaled && !keep_pairs && beta_zero && mma_supported(pb, xt, ot, kind)) return route::mma;
+    // dense complex (IQ) data: batch tiles on windows of plain samples, forward and adjoint
+    if (ot == FFDAS_C_32F && iq_supported(pb, kind)) return route::iq;
+    // das_sparse: a lane per list entry where the lists are long enough
+    if (ot == FFDAS_R_32F && entries_supported(pb, kind)) return route::entries;
+    return route::pairs;
+}
+
+// Bytes of the pair buffer that a forward call on this handle would fill and
+// its adjoint read: 0 where one of them does without pair rows.
+ffdas_error_t kept_pair_bytes(const ffdas_context &h, const das_call &a, bool scaled, size_t *bytes) {
+    *bytes = 0;
+    const ffdas_tensor_desc &xd = *a.x_desc, &od = *a.out_desc;
+    const int batch = xd.ndim == 4 ? (int)xd.dims[0] : 1;
+    const int kind = select_storage(xd.dtype, od.dtype, a.compute_type, batch);
+    das_problem pb;
+    if (kind < 0 || !fits_int32_indexing(xd) || !fits_int32_indexing(od) || make_problem(xd, od, pb) != FFDAS_SUCCESS)
+        return FFDAS_SUCCESS;   // the call itself reports it
+    pb.sparse = a.sparse;
+    pb.n_events = a.sparse ? a.sparse_count : pb.S;
+    // (the adjoint computes in the default type)
+    if (kind != select_storage(xd.dtype, od.dtype, FFDAS_COMPUTE_DEFAULT, batch) ||
+        forward_route(h, pb, xd.dtype, od.dtype, kind, scaled, true, true) != route::pairs)
+        return FFDAS_SUCCESS;
+    return pair_buffer_bytes(xd, a.compute_type, bytes);
+}
+
 ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     const ffdas_tensor_desc &xd = *a.x_desc;
     const ffdas_tensor_desc &od = *a.out_desc;
@@ -519,36 +566,27 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         FFDAS_TRY(channel_gain(h, pb, &g, &gb));
     }
 
+    double br = 0.0, bi = 0.0;
+    int bz = 1;
+    read_beta(od.dtype, a.beta, br, bi, bz);
+    const route way =
+        forward_route(h, pb, xd.dtype, od.dtype, kind, h.chan_scale != nullptr, h.pair_buf != nullptr, bz != 0);
+
     // ---- small problems: the whole call as one launch straight from x ----
-    // (it reads x in place, so not with a channel scale, which the ingest applies)
-    if (!h.chan_scale && direct_supported(pb, xd.dtype, od.dtype, kind)) {
+    if (way == route::direct) {
         const bool asked = h.has_config && h.config.variant == 5;
-        const bool planner = !h.has_config || h.config.variant == 0;
-        const int64_t units = pb.V * pb.C * (int64_t)pb.S * pb.B;
-        if (asked || (planner && units <= (pb.B == 1 ? kDirectUnits : kDirectUnitsBatched) &&
-                      !(!h.has_config && pb.B == 1 && pb.V >= kDirectFrameVoxels && units >= kDirectFrameUnits))) {
-            double br = 0.0, bi = 0.0;
-            int bz = 1;
-            read_beta(od.dtype, a.beta, br, bi, bz);
-            return launch_direct(h, pb, xd.dtype, a.x, a.srcpos, a.srcdir, a.dstpos, a.offsets, a.weights,
-                                 static_cast<float *>(a.out), br, bz, asked ? h.config.batch_tile : 0,
-                                 asked ? h.config.tile_x : 0);
-        }
+        return launch_direct(h, pb, xd.dtype, a.x, a.srcpos, a.srcdir, a.dstpos, a.offsets, a.weights,
+                             static_cast<float *>(a.out), br, bz, asked ? h.config.batch_tile : 0,
+                             asked ? h.config.tile_x : 0);
     }
 
     // ---- large half-precision batches: tensor cores, straight from x ----
-    // (not with a pair buffer to fill, a channel scale or a prior image to keep)
-    if (!h.has_config && !h.chan_scale && !h.pair_buf && mma_supported(pb, xd.dtype, od.dtype, kind)) {
-        double br = 0.0, bi = 0.0;
-        int bz = 1;
-        read_beta(od.dtype, a.beta, br, bi, bz);
-        if (bz) return launch_mma(h, pb, a, static_cast<float *>(a.out));
-    }
+    if (way == route::mma) return launch_mma(h, pb, a, static_cast<float *>(a.out));
 
     // ---- dense complex (IQ) data without a schedule: batch tiles on windows of
-    // plain samples (das_iq.cuh).  (A pair buffer stays unfilled: its adjoint
-    // reads no pairs.)
-    if (!h.has_config && od.dtype == FFDAS_C_32F && iq_supported(pb, kind)) {
+    // plain samples (das_iq.cuh).  (A pair buffer stays unfilled: the adjoint of
+    // such a call reads no pairs.)
+    if (way == route::iq) {
         const float *gain = nullptr;
         int gain_bstride = 0;
         FFDAS_TRY(channel_gain(h, pb, &gain, &gain_bstride));
@@ -563,15 +601,16 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         gp.wavenum = a.wavenum;
         gp.out = a.out;
         gp.out_bstride = pb.out_bstride;
-        read_beta(od.dtype, a.beta, gp.beta_re, gp.beta_im, gp.beta_zero);
+        gp.beta_re = br; gp.beta_im = bi; gp.beta_zero = bz;
         h.last = ffdas_kernel_info_t{};
         return launch_iq(h, pb, xd.dtype, kind, a.x, gain, gain_bstride, gp, IW.get<void>());
     }
 
     // ---- das_sparse without a schedule: a lane per list entry on staged sample
     // windows (das_entries.cuh) where the lists are long enough; the gather
-    // kernel else.  (A pair buffer stays unfilled: its adjoint reads no pairs.)
-    if (!h.has_config && od.dtype == FFDAS_R_32F && entries_supported(pb, kind)) {
+    // kernel else.  (A pair buffer stays unfilled: the adjoint, which does read
+    // pairs, builds them.)
+    if (way == route::entries) {
         const float *gain = nullptr;
         int gain_bstride = 0;
         FFDAS_TRY(channel_gain(h, pb, &gain, &gain_bstride));
@@ -586,7 +625,7 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         gp.sparse_idx = a.sparse_indices;
         gp.out = a.out;
         gp.out_bstride = pb.out_bstride;
-        read_beta(od.dtype, a.beta, gp.beta_re, gp.beta_im, gp.beta_zero);
+        gp.beta_re = br; gp.beta_im = bi; gp.beta_zero = bz;
         h.last = ffdas_kernel_info_t{};
         h.last.storage = kind;
         h.mark_start();
@@ -672,7 +711,7 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     gp.wavenum = a.wavenum;
     gp.out = a.out;
     gp.out_bstride = pb.out_bstride;
-    read_beta(od.dtype, a.beta, gp.beta_re, gp.beta_im, gp.beta_zero);
+    gp.beta_re = br; gp.beta_im = bi; gp.beta_zero = bz;
 
     const int64_t tiles = (int64_t)gp.n0 * gp.n1 * n2;
     const int bchunks = (pb.B + s.BT - 1) / s.BT;

@@ -4,6 +4,7 @@
 #include <cstring>
 
 #include "core.h"
+#include "das_problem.h"
 
 namespace {
 
@@ -49,44 +50,75 @@ ffdas_error_t read_image(reader &r, ffdas_tensor_desc &d) {
     return ffdas_type_size(d.dtype) ? FFDAS_SUCCESS : FFDAS_ERROR_UNSUPPORTED_TYPE;
 }
 
+// A forward call unpacked; its descriptors stay here.
+struct forward_args {
+    ffdas_handle_t h = nullptr;
+    uintptr_t stream = 0;
+    ffdas_tensor_desc xd, od;
+    ffdas::das_call a;
+    const float *scale = nullptr;
+    int64_t scale_count = 0;
+    void *pairs = nullptr;
+    size_t pair_bytes = 0;
+
+    ffdas_error_t read(const int64_t *q, int64_t n) {
+        if (!q) return FFDAS_ERROR_NULL_POINTER;
+        reader r{q, n};
+        h = r.ptr<ffdas_context>();
+        if (!h) return FFDAS_ERROR_INVALID_HANDLE;
+        stream = (uintptr_t)r.next();
+        a.srcpos = r.ptr<const float>();
+        a.srcdir = r.ptr<const float>();
+        a.wavenum = r.real();
+        a.x = r.ptr<const void>();
+        FFDAS_TRY(read_x(r, xd));
+        a.dstpos = r.ptr<const float>();
+        a.offsets = r.ptr<const float>();
+        a.weights = r.ptr<const float>();
+        a.sparse_count = (int)r.next();
+        a.sparse_indices = r.ptr<const int>();
+        a.out = r.ptr<void>();
+        od.dtype = (ffdas_datatype_t)r.next();
+        a.compute_type = (ffdas_compute_type_t)r.next();
+        a.alg = (ffdas_alg_t)r.next();
+        scale = r.ptr<const float>();
+        scale_count = r.next();
+        pairs = r.ptr<void>();
+        pair_bytes = (size_t)r.next();
+        a.sparse = r.next() != 0;
+        FFDAS_TRY(read_image(r, od));
+        a.x_desc = &xd;
+        a.out_desc = &od;
+        return FFDAS_SUCCESS;
+    }
+};
+
 }  // namespace
 
 extern "C" {
 
 ffdas_error_t ffdas_das_call(const int64_t *q, int64_t n) {
-    if (!q) return FFDAS_ERROR_NULL_POINTER;
-    reader r{q, n};
-    ffdas_handle_t h = r.ptr<ffdas_context>();
-    if (!h) return FFDAS_ERROR_INVALID_HANDLE;
-    const uintptr_t stream = (uintptr_t)r.next();
-    const float *srcpos = r.ptr<const float>(), *srcdir = r.ptr<const float>();
-    const float wavenum = r.real();
-    const void *x = r.ptr<const void>();
-    ffdas_tensor_desc xd, od;
-    FFDAS_TRY(read_x(r, xd));
-    const float *dstpos = r.ptr<const float>(), *offsets = r.ptr<const float>(), *weights = r.ptr<const float>();
-    const int count = (int)r.next();
-    const int *idx = r.ptr<const int>();
-    void *out = r.ptr<void>();
-    od.dtype = (ffdas_datatype_t)r.next();
-    const ffdas_compute_type_t ct = (ffdas_compute_type_t)r.next();
-    const ffdas_alg_t alg = (ffdas_alg_t)r.next();
-    const float *scale = r.ptr<const float>();
-    const int64_t scale_count = r.next();
-    void *pairs = r.ptr<void>();
-    const size_t pair_bytes = (size_t)r.next();
-    const bool sparse = r.next() != 0;
-    FFDAS_TRY(read_image(r, od));
-    FFDAS_TRY(ffdas_set_stream(h, stream));
-    if (scale) FFDAS_TRY(ffdas_set_channel_scale(h, scale, scale_count));
-    ffdas_error_t e = pairs ? ffdas_set_pair_buffer(h, pairs, pair_bytes) : FFDAS_SUCCESS;
+    forward_args f;
+    FFDAS_TRY(f.read(q, n));
+    const ffdas::das_call &a = f.a;
+    FFDAS_TRY(ffdas_set_stream(f.h, f.stream));
+    if (f.scale) FFDAS_TRY(ffdas_set_channel_scale(f.h, f.scale, f.scale_count));
+    ffdas_error_t e = f.pairs ? ffdas_set_pair_buffer(f.h, f.pairs, f.pair_bytes) : FFDAS_SUCCESS;
     if (e == FFDAS_SUCCESS)
-        e = sparse ? ffdas_das_sparse(h, srcpos, srcdir, wavenum, &xd, x, dstpos, offsets, weights, count, idx, nullptr,
-                                      &od, out, ct, alg)
-                   : ffdas_das(h, srcpos, srcdir, wavenum, &xd, x, dstpos, offsets, weights, nullptr, &od, out, ct, alg);
-    if (pairs) ffdas_set_pair_buffer(h, nullptr, 0);
-    if (scale) ffdas_set_channel_scale(h, nullptr, 0);
+        e = a.sparse ? ffdas_das_sparse(f.h, a.srcpos, a.srcdir, a.wavenum, &f.xd, a.x, a.dstpos, a.offsets, a.weights,
+                                        a.sparse_count, a.sparse_indices, nullptr, &f.od, a.out, a.compute_type, a.alg)
+                     : ffdas_das(f.h, a.srcpos, a.srcdir, a.wavenum, &f.xd, a.x, a.dstpos, a.offsets, a.weights, nullptr,
+                                 &f.od, a.out, a.compute_type, a.alg);
+    if (f.pairs) ffdas_set_pair_buffer(f.h, nullptr, 0);
+    if (f.scale) ffdas_set_channel_scale(f.h, nullptr, 0);
     return e;
+}
+
+ffdas_error_t ffdas_das_call_pair_bytes(const int64_t *q, int64_t n, size_t *bytes) {
+    if (!bytes) return FFDAS_ERROR_NULL_POINTER;
+    forward_args f;
+    FFDAS_TRY(f.read(q, n));
+    return ffdas::kept_pair_bytes(*f.h, f.a, f.scale || f.h->chan_scale, bytes);
 }
 
 ffdas_error_t ffdas_das_backward_call(const int64_t *q, int64_t n) {

@@ -54,6 +54,7 @@ ffdas_error_t make_problem(const ffdas_tensor_desc &x, const ffdas_tensor_desc &
 int select_storage(ffdas_datatype_t xt, ffdas_datatype_t ot, ffdas_compute_type_t ct, int batch);
 
 ffdas_error_t das_forward(ffdas_context &h, const das_call &a);
+ffdas_error_t kept_pair_bytes(const ffdas_context &h, const das_call &a, bool scaled, size_t *bytes);
 
 // Pairs per row, rounded so every row starts 16-byte aligned for both pair
 // sizes (the TMA tensor map needs 16-byte row strides).

@@ -177,12 +177,16 @@ def _check_spatial(dstpos, offsets, weights, sparse_indices=None):
     return spatial
 
 
+_PAIR_WORD = 27   # place of the pair buffer among ffdas_das_call's packed values
+
+
 def _needs_grad(*ts) -> bool:
     return torch.is_grad_enabled() and any(torch.is_tensor(t) and t.requires_grad for t in ts)
 
 
 def _run(x, srcpos, dstpos, offsets, weights, sparse_indices, *, srcdir, wavenum, algorithm,
-         use_fp16, use_bf16, channels_trailing, out, channel_scale=None, host_chunks=None, pair_buffer=None):
+         use_fp16, use_bf16, channels_trailing, out, channel_scale=None, host_chunks=None, keep_pairs=False):
+    """One forward call.  With keep_pairs returns (image, pair buffer for the backward or None)."""
     spatial = _check_spatial(dstpos, offsets, weights, sparse_indices)
     xt = _to_torch(x)
     if xt.ndim not in (3, 4):
@@ -236,9 +240,18 @@ def _run(x, srcpos, dstpos, offsets, weights, sparse_indices, *, srcdir, wavenum
                         _FFDAS_DTYPE[xt.dtype], *_x_layout(xt, channels_trailing), ptr(dstpos_t), ptr(offsets_t),
                         ptr(weights_t), idx_t.shape[0] if idx_t is not None else 0, ptr(idx_t), ptr(out_t),
                         _FFDAS_DTYPE.get(out_t.dtype, DataType.R_32F), ctype, int(algorithm), ptr(scale_t),
-                        scale_t.numel() if scale_t is not None else 0, *(pair_buffer or (0, 0)), idx_t is not None,
+                        scale_t.numel() if scale_t is not None else 0, 0, 0, idx_t is not None,
                         len(od), *od, *out_t.stride()])
+        pairs = None
+        if keep_pairs:
+            nbytes = ctypes.c_size_t()
+            _lib.check(L.ffdas_das_call_pair_bytes(q.buffer_info()[0], len(q), ctypes.byref(nbytes)))
+            if nbytes.value:
+                pairs = torch.empty(nbytes.value, dtype=torch.uint8, device=dev)
+                q[_PAIR_WORD], q[_PAIR_WORD + 1] = pairs.data_ptr(), nbytes.value
         _lib.check(L.ffdas_das_call(q.buffer_info()[0], len(q)))
+        if keep_pairs:
+            return out_t, pairs
         if out is not None:
             return out
         return _from_torch_like(out_t, x)

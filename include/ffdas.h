@@ -346,6 +346,12 @@ FFDAS_API ffdas_error_t ffdas_das_pair_bytes(ffdas_tensor_desc_t x_desc, ffdas_c
  * cleared after the call. */
 FFDAS_API ffdas_error_t ffdas_das_call(const int64_t *q, int64_t n);
 
+/* New: bytes of the pair buffer that the call packed in q (its pair buffer and
+ * bytes unread) would fill and ffdas_das_backward read; 0 where the forward or
+ * the adjoint does without pair rows (small calls, dense complex data, long
+ * das_sparse lists), so that no buffer need be held for them. */
+FFDAS_API ffdas_error_t ffdas_das_call_pair_bytes(const int64_t *q, int64_t n, size_t *bytes);
+
 /* New: the same for ffdas_das_backward:
  *   handle, stream, srcpos, srcdir, wavenum, x, x dtype, x ndim, four dims, four
  *   strides, dstpos, offsets, weights, sparse_count, sparse_indices, grad_out,

@@ -322,6 +322,24 @@ def test_tensor_core_batches_channels_trailing_view_and_non_finite_values():
     assert oracle.rel_l2(got[both], clean[both]) < TOL
 
 
+@pytest.mark.parametrize("kind,variant,kept", [("staged", 2, True), ("batch", 2, True), ("lists", 1, True), ("direct", 5, False),
+                                               ("iq", 2, False), ("entries", 9, False)])
+def test_pair_buffer_only_where_the_backward_reads_it(kind, variant, kept):
+    B, C, S, n, dtype = dict(staged=(1, 1200, 4, 4, torch.float32), batch=(33, 20, 3, 3, torch.float16),
+                             lists=(1, 40, 8, 4, torch.float32), direct=(1, 40, 3, 3, torch.float32),
+                             iq=(2, 20, 3, 3, torch.complex64), entries=(4, 1000, 4, 4, torch.float32))[kind]
+    x, src, dst, offs, w = _problem(B, C, S, 512, 131, 67, dtype=dtype, n=n)
+    x, src, dst, offs, w = [t.to(DEV).requires_grad_(i == 3) for i, t in enumerate((x, src, dst, offs, w))]
+    if kind in ("lists", "entries"):
+        out = ffdas_b200.das_sparse(x, src, dst, offs, w, _lists(S, n, (131, 67), seed=1)[0].to(DEV))
+    else:
+        out = ffdas_b200.das(x, src, dst, offs, w)
+    assert _info()["variant"] == variant
+    assert (out.grad_fn.pairs is not None) == kept
+    out.backward(torch.ones_like(out))
+    assert torch.isfinite(offs.grad).all() and offs.grad.abs().max() > 0
+
+
 @pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9, 16, 17, 31, 32])
 @pytest.mark.parametrize("S", [33, 97])
 def test_select_sizes(k, S):
