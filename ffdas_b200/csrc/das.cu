@@ -474,7 +474,7 @@ static route forward_route(const ffdas_context &h, const das_problem &pb, ffdas_
         const bool planner = !h.has_config || h.config.variant == 0;
         const int64_t units = pb.V * pb.C * (int64_t)pb.S * pb.B;
         if (asked || (planner && units <= (pb.B == 1 ? kDirectUnits : kDirectUnitsBatched) &&
-                      !(!h.has_config && pb.B == 1 && pb.V >= kDirectFrameVoxels && units >= kDirectFrameUnits)))
+                      !(!h.has_config && pb.B == 1 && staged_frame(pb.V, pb.S, units))))
             return route::direct;
     }
     if (h.has_config) return route::pairs;
@@ -651,7 +651,7 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     // without a schedule the staged kernels' tile shape and window width follow
     // the geometry (das_tile_plan.cuh)
     const bool staged_ok = staged_supported(pb, kind) && od.dtype == FFDAS_R_32F;
-    schedule s = plan_schedule(h, pb, kind, staged_ok);
+    const schedule s = plan_schedule(h, pb, kind, staged_ok);
     // (batch tiles and the 512-voxel tiles of one item read a plan; the 256-voxel
     // kernel of a batch that cannot have TMA boxes does not)
     const bool planned = s.variant == 2 && !h.has_config && (s.BT > 1 || s.T0 * s.T1 * s.T2 == 512);
@@ -659,11 +659,6 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     const int64_t plan_tiles = plan_tile && pb.C > 0 ? plan_max_tiles(pb, plan_tile) : 0;
     void *const plan = plan_tiles > 0 && plan_tiles <= INT32_MAX ? static_cast<char *>(Pbase) + pair_bytes + 64 : nullptr;
     if (plan) {
-        // one item: event chunks of 4 run three CTAs per SM, of 8 two (1024 channels,
-        // 16 events, 128^3 voxels: 7.3 against 8.1 ms; 484 channels, 7 events, 44 x
-        // 59 x 59: 435 against 518 us; a 300 x 256 frame of 16 events, where 8 save
-        // half the passes, 194 against 180)
-        if (pb.B == 1) s.SC = std::min(s.SC, 4);
         const plan_params own = make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, npad, plan_tile,
                                           s.BT > 1 ? kPlanBatch : kPlanForward, plan);
         // pair rows kept for a backward: the adjoint's plan beside the forward's
@@ -770,15 +765,31 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
             csplit = (pb.C + chunk - 1) / chunk;
             gp.cchunk = csplit > 1 ? chunk : 0;
         }
+        // One item on a plan: event chunks of 4 or 8 for each window width.  Eight save
+        // half the passes and their geometry; four let three CTAs of the 32-sample
+        // instance share an SM where eight let two (the 64-sample instance has two
+        // either way).  So four for the narrow windows of more CTAs than two per SM,
+        // counted in full slices, and where eight would only add empty places.  SC 4 and
+        // 8, us: narrow, 1024 channels, 16 events, 128^3 voxels 7300 and 8100; 484, 7,
+        // 44 x 59 x 59 (352 CTAs) 420 and 474; 72, 8, 300 x 250 pixels (169) 64 and 58;
+        // wide, 128, 16, 300 x 250 172 and 161; 96, 8, 350 x 240 72 and 65; with empty
+        // places 128, 10, 350 x 240 134 and 149.
+        int SC = s.SC, SC_wide = s.SC;
+        if (plan && pb.B == 1 && pb.n_events > 4) {
+            const bool full = (pb.n_events + 7) / 8 * 8 == (pb.n_events + 3) / 4 * 4;
+            const int64_t work = plan_min_tiles(pb, plan_tile) * pb.C / (gp.cchunk ? gp.cchunk : std::max(pb.C, 1));
+            SC_wide = full ? 8 : 4;
+            SC = full && work <= 2 * (int64_t)std::max(h.sm_count, 1) ? 8 : 4;
+        }
         h.last.variant = 2;
         h.last.batch_tile = s.BT;
-        h.last.event_chunk = s.SC;
+        h.last.event_chunk = SC;
         h.last.grid = tiles * bchunks_st * csplit;
         // (plan,) ingest, (image preparation,) delay-and-sum, (the width not taken)
         h.last.kernels = (csplit > 1 ? 3 : 2) + (gp.plan ? (s.BT == 1 ? 2 : 1) : 0);
         if (bchunks_st > 65535) return FFDAS_ERROR_DIMS_TOO_LARGE;
         h.mark_start();
-        const ffdas_error_t err = launch_staged(h, pb, kind, gp, s.SC, s.WB, s.BT, s.copy,
+        const ffdas_error_t err = launch_staged(h, pb, kind, gp, SC, SC_wide, s.WB, s.BT, s.copy,
                                                 dim3((unsigned)tiles, (unsigned)bchunks_st, (unsigned)csplit));
         h.mark_stop();
         return err;

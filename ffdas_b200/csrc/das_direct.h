@@ -10,13 +10,23 @@ namespace ffdas {
 // units (measured on B200: 15 us against 18-27 us staged for a 4.2e6-unit
 // plane-wave frame, 39 us against 49 us at 2.7e7 units), batches up to 2^22
 // (the staged batch tiles share each tap's delay over the items; the direct
-// kernel only shares the geometry).  Without a schedule a frame of 2^16 voxels
-// and 2^24 units is staged: it fills the tiles (320 x 216 pixels, 70 channels, 4
-// events 94 us direct, 55 staged; 256 x 256, 128, 2: 57 and 48; with 1 event 37 in
-// both; 149 x 215, 102, 5: 62 direct, 69 staged).
+// kernel only shares the geometry).
 constexpr int64_t kDirectUnits = int64_t(1) << 25;
-constexpr int64_t kDirectFrameVoxels = int64_t(1) << 16, kDirectFrameUnits = int64_t(1) << 24;
 constexpr int64_t kDirectUnitsBatched = int64_t(1) << 22;
+
+// Frames among them that are staged without a schedule: 2^24 units on 2^16 voxels
+// fill the staged tiles.  Not two events, whose passes of four are half empty; and
+// five or more only past the voxels that get eight threads each in the direct
+// kernel's two waves (148 SMs x 2048 threads): with four its chains double.  Direct
+// and staged, us per call: 400 x 256 pixels, 64 channels, 4 events 57 and 38; 96, 3:
+// 71 and 52; 192, 1: 58 and 42; 48, 6: 64 and 46; 256 x 256, 128, 3: 51 and 42;
+// 300 x 250, 48, 5: 33 and 46; 40, 6: 33 and 42; 63, 5: 41 and 53; two events, 300 x
+// 250, 192 channels: 58 and 123 (windows that overflow); 400 x 256, 90: 49 and 52.
+constexpr int64_t kFrameUnits = int64_t(1) << 24, kFrameVoxels = int64_t(1) << 16;
+constexpr int64_t kEightThreadVoxels = int64_t(2) * 148 * 2048 / 8;
+inline bool staged_frame(int64_t V, int S, int64_t units) {
+    return units >= kFrameUnits && V >= kFrameVoxels && S != 2 && (S <= 4 || V > kEightThreadVoxels);
+}
 
 // Real channel data (f32, f16, bf16) into f32 output, dense.
 bool direct_supported(const das_problem &pb, ffdas_datatype_t xt, ffdas_datatype_t ot, int kind);

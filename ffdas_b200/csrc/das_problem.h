@@ -79,9 +79,10 @@ bool staged_batch_supported();
 ffdas_error_t launch_scale_image(ffdas_context &h, const das_problem &pb, float *out, float beta, int beta_zero);
 // BT > 1: batch tiles of BT items per CTA (256-voxel tiles, SC * BT <= 32).
 // With gp.plan set the tile shape and the window width come from the plan
-// made there; grid.x is then plan_max_tiles().
+// made there; grid.x is then plan_max_tiles(), and the 64-sample instance of one
+// item takes event chunks of SC_wide.
 ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp, int SC,
-                            int WB, int BT, int copy, dim3 grid);
+                            int SC_wide, int WB, int BT, int copy, dim3 grid);
 
 // Most tiles of any candidate shape of `tile_voxels` voxels; 0 when the grid
 // admits none (then no plan).

@@ -266,7 +266,7 @@ static ffdas_error_t launch_staged_width(ffdas_context &h, const das_problem &pb
                                          int SC, int WB, int BT, int copy, dim3 grid);
 
 ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp, int SC,
-                            int WB, int BT, int copy, dim3 grid) {
+                            int SC_wide, int WB, int BT, int copy, dim3 grid) {
     if (gp.cchunk) {   // channel slices add into the image: prepare it (beta * out, or 0)
         if (grid.z < 2) return FFDAS_ERROR_INTERNAL;
         dim3 sg((unsigned)((pb.V + 255) / 256), (unsigned)std::min(pb.B, 65535));
@@ -278,7 +278,7 @@ ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, c
     if (gp.plan && BT == 1 && gp.T0 * gp.T1 * gp.T2 != 2 * kStConsumers) return FFDAS_ERROR_INTERNAL;
     if (!gp.plan || BT > 1) return launch_staged_width(h, pb, kind, gp, SC, BT > 1 && gp.plan ? 64 : WB, BT, copy, grid);
     FFDAS_TRY(launch_staged_width(h, pb, kind, gp, SC, 32, BT, copy, grid));
-    return launch_staged_width(h, pb, kind, gp, SC, 64, BT, copy, grid);
+    return launch_staged_width(h, pb, kind, gp, SC_wide, 64, BT, copy, grid);
 }
 
 static ffdas_error_t launch_staged_width(ffdas_context &h, const das_problem &pb, int kind, const gather_params &gp,
