@@ -609,13 +609,13 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     // ---- das_sparse without a schedule: a lane per list entry on staged sample
     // windows (das_entries.cuh) where the lists are long enough; the gather
     // kernel else.  (A pair buffer stays unfilled: the adjoint, which does read
-    // pairs, builds them.)
-    if (way == route::entries) {
-        const float *gain = nullptr;
-        int gain_bstride = 0;
-        FFDAS_TRY(channel_gain(h, pb, &gain, &gain_bstride));
-        workspace EW(h);
-        FFDAS_TRY(EW.alloc(entries_workspace(pb)));
+    // pairs, builds them.)  The sorted entries take more memory than the lists;
+    // where it cannot be had, the kernels on pair rows compute the call.
+    const float *gain = nullptr;
+    int gain_bstride = 0;
+    FFDAS_TRY(channel_gain(h, pb, &gain, &gain_bstride));
+    workspace EW(h);
+    if (way == route::entries && EW.alloc(entries_workspace(pb, xd.dtype, kind, a.x, gain)) == FFDAS_SUCCESS) {
         gather_params gp;
         std::memset(&gp, 0, sizeof(gp));
         gp.C = pb.C; gp.S = pb.S; gp.n_events = pb.n_events; gp.B = pb.B; gp.V = pb.V;

@@ -109,20 +109,20 @@ static int64_t entries_tiles(const das_problem &pb, const en_params &e) {
     return (int64_t)e.n0 * e.n1 * ((pb.D2 + e.T2 - 1) / e.T2);
 }
 
-size_t entries_workspace(const das_problem &pb) {
+size_t entries_workspace(const das_problem &pb, ffdas_datatype_t xt, int kind, const void *x, const float *gain) {
     gather_params gp;
     std::memset(&gp, 0, sizeof(gp));
     const en_params e = make_params(pb, gp);
     const int64_t tiles = entries_tiles(pb, e);
-    return rows_bytes(pb) + (size_t)tiles * (sizeof(en_tile) + sizeof(en_slot) * e.slots_cap + sizeof(en_entry) * kEnTile * e.n);
+    return (in_place(pb, xt, kind, x, gain) ? 0 : rows_bytes(pb)) + (size_t)tiles * (sizeof(en_tile) + sizeof(en_slot) * e.slots_cap + sizeof(en_entry) * kEnTile * e.n);
 }
 
-// Sorts the lists of every tile into the workspace.
-static ffdas_error_t launch_sort(ffdas_context &h, const das_problem &pb, en_params &e, void *ws, int64_t *tiles) {
+// Sorts the lists of every tile into `ws`.
+static ffdas_error_t launch_sort(ffdas_context &h, const das_problem &pb, en_params &e, char *ws, int64_t *tiles) {
     *tiles = entries_tiles(pb, e);
     if (*tiles > INT32_MAX) return FFDAS_ERROR_DIMS_TOO_LARGE;
     static_assert(sizeof(en_tile) == 256 && sizeof(en_slot) == 16 && sizeof(en_entry) == 16, "workspace layout");
-    char *w = static_cast<char *>(ws) + rows_bytes(pb);
+    char *w = ws;
     e.entries = reinterpret_cast<en_entry *>(w);
     w += (size_t)*tiles * sizeof(en_entry) * kEnTile * e.n;
     e.tiles = reinterpret_cast<en_tile *>(w);
@@ -172,7 +172,7 @@ ffdas_error_t launch_entries(ffdas_context &h, const das_problem &pb, ffdas_data
     bool copied = false;
     FFDAS_TRY(make_rows(h, pb, xt, kind, x, gain, gain_bstride, ws, e.rows, &copied));
     int64_t tiles = 0;
-    FFDAS_TRY(launch_sort(h, pb, e, ws, &tiles));
+    FFDAS_TRY(launch_sort(h, pb, e, static_cast<char *>(ws) + (copied ? rows_bytes(pb) : 0), &tiles));
     gp.T0 = e.T0; gp.T1 = e.T1; gp.T2 = e.T2; gp.n0 = e.n0; gp.n1 = e.n1;
     const int slices = entries_slices(h, pb, tiles * pb.B, 3, 16, &gp.cchunk);
     if (gp.cchunk)

@@ -136,9 +136,10 @@ ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call
 
 // das_sparse on sorted list entries (csrc/das_entries.cuh): real storage kinds,
 // f32 output, lists of at most 64 entries over at most 480 events; no pair
-// rows.  ws is entries_workspace() bytes; gain as in the ingest.
+// rows.  ws is entries_workspace() bytes (16 a list place, and a copy of x where
+// its rows cannot be read in place); gain as in the ingest.
 bool entries_supported(const das_problem &pb, int kind);
-size_t entries_workspace(const das_problem &pb);
+size_t entries_workspace(const das_problem &pb, ffdas_datatype_t xt, int kind, const void *x, const float *gain);
 ffdas_error_t launch_entries(ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt, int kind, const void *x,
                              const float *gain, int gain_bstride, gather_params gp, void *ws);
 

@@ -276,6 +276,23 @@ def test_sorted_entries_strided_data():
     assert torch.linalg.norm(got - ref) < 1e-6 * torch.linalg.norm(ref)
 
 
+def test_sorted_entries_without_memory_fall_back_to_pair_rows():
+    # FP32 rows that are read in place take no room for a copy; a workspace that does
+    # not fit leaves the call to the kernels on pair rows, as before
+    x, src, dst, offs, _ = _problem(4, 1000, 4, 512, 131, 67, n=4)
+    idx, w = _lists(4, 4, (131, 67), seed=2)
+    args = _dev(x, src, dst, offs, w, idx)
+    ref = ffdas_b200.das_sparse(*args)
+    assert _info()["variant"] == 9
+    _lib.load().ffdas_debug_fail_alloc_after(1)
+    try:
+        got = ffdas_b200.das_sparse(*args)
+        assert _info()["variant"] != 9
+    finally:
+        _lib.load().ffdas_debug_fail_alloc_after(0)
+    assert oracle.rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < TOL
+
+
 def test_sorted_entries_non_finite_delay_stays_in_its_voxel():
     x, src, dst, offs, _ = _problem(4, 1000, 4, 512, 131, 67, n=4)
     idx, w = _lists(4, 4, (131, 67), seed=2)
