@@ -1515,6 +1515,39 @@ __global__ void __launch_bounds__(kStThreads, SC >= 8 ? 2 : 3) das_staged2_kerne
                         }
                         uint32_t k0p[SC];
                         load_meta<SC>(sm.meta, stage, cl, k0p);
+                        // Every window of the channel too wide (events past the chunk read
+                        // the zero pair): no test per tap, and the pairs of two events are
+                        // loaded before the first is used (186 channels, 12 events, 359 x 95
+                        // pixels: 310 us one by one, 225 two, 256 four events at a time,
+                        // which spills).
+                        bool rows = true;
+#pragma unroll
+                        for (int j = 0; j < SC; j++) rows &= k0p[j] == kOvf || j >= sc;
+                        if (rows) {
+                            constexpr int G = SC < 2 ? SC : 2;
+                            const st *r0 = Pg + (((int64_t)cx.b * p.C + c) * p.S + e0) * p.npad;
+                            const uint32_t npad = (uint32_t)p.npad;
+#pragma unroll
+                            for (int j0 = 0; j0 < SC; j0 += G) {
+                                st pa[G], pb[G];
+                                float2 t2[G];
+#pragma unroll
+                                for (int i = 0; i < G; i++) {
+                                    const float2 o2 = ofs2[j0 + i];
+                                    const tau_split ta = split_tau(__fmaf_rn(ga.rsq, ga.rinv, o2.x));
+                                    const tau_split tb = split_tau(__fmaf_rn(gb.rsq, gb.rinv, o2.y));
+                                    const uint32_t row = (uint32_t)min(j0 + i, sc - 1) * npad;   // < 2^26
+                                    pa[i] = r0[row + min(ta.k, kmax_pair)];
+                                    pb[i] = r0[row + min(tb.k, kmax_pair)];
+                                    t2[i] = make_float2(ta.t, tb.t);
+                                }
+#pragma unroll
+                                for (int i = 0; i < G; i++)
+                                    acc2 = __ffma2_rn(w2[j0 + i], make_float2(pair_traits<K>::tap(pa[i], t2[i].x),
+                                                                              pair_traits<K>::tap(pb[i], t2[i].y)), acc2);
+                            }
+                            continue;
+                        }
                         const unsigned char *slots = sm.ring + stage * SG::stage_bytes + (cl * SC) * SG::bytes;
 #pragma unroll
                         for (int j = 0; j < SC; j++) {

@@ -368,3 +368,18 @@ def test_select_sizes(k, S):
     order = torch.sort(w, dim=0, descending=True, stable=True)[1][:k]
     assert torch.equal(idx.cpu().long(), order)
     assert torch.equal(sw.cpu(), w.gather(0, order)) and torch.equal(so.cpu(), o.gather(0, order))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.int16])
+@pytest.mark.parametrize("S", [1, 2, 3, 5, 7, 8, 9])
+def test_rows_where_every_window_is_too_wide(dtype, S):
+    # pixels 24 samples apart along both axes: each channel's windows all overflow, or
+    # some of an event chunk do (the tile's corner), with chunks that are not full
+    C = 40
+    x, src, dst, offs, w = _problem(1, C, S, 700, 40, 110, (24.0, 24.0), seed=S, dtype=torch.float32)
+    x = (x * 300).round().to(dtype) if dtype == torch.int16 else x.to(dtype)
+    rep = 1 + (1 << 25) // (C * S * 4400)   # past the direct kernel
+    ref = rep * _oracle(x.float(), src, dst, offs, w)
+    got = ffdas_b200.das(*_dev(x.repeat(1, rep, 1, 1), src.repeat(rep, 1), dst, offs, w))
+    assert _info()["variant"] == 2
+    assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL
