@@ -196,9 +196,8 @@ __device__ __forceinline__ void iq_event_phases(const iq_params &q, bool active,
         E[j] = (active && j < sc) ? iq_phase(ofs[j], q.turn_hi, q.turn_lo) : make_float2(0.f, 0.f);
 }
 
-// apply_directivity; an excluded channel has no factor either: one whose
-// position is not finite (its distance and factor are NaN) is excluded too, and
-// adds nothing.
+// apply_directivity; an excluded channel has no factor either: one infinitely far
+// away (its distance and factor are NaN) is excluded too, and adds nothing.
 __device__ __forceinline__ void iq_directivity(recv_geom &g, float2 &R, const staged_ctx &cx, float4 c, float4 dir) {
     apply_directivity(g, cx.vx, cx.vy, cx.vz, c.x, c.y, c.z, dir);
     if (g.rsq == 1e30f) R = make_float2(0.f, 0.f);

@@ -254,6 +254,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) das_mma_kernel(const __grid_co
     int since = 0;          // (channel, event) pairs since the accumulators were drained
     uint32_t drains = 0;
     bool fresh = true;      // nothing accumulated since the last drain
+    bool spoiled = false;   // poison (of every voxel) since the last drain
     bool dead = false, first_out = true;
     int prev = -1;          // column this thread wrote into its buffer last time
     bool odd = false;       // a value that is not finite went into the image
@@ -298,6 +299,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) das_mma_kernel(const __grid_co
         }
         drains++;
         fresh = true;
+        spoiled = false;
         since = 0;
     };
 
@@ -311,7 +313,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) das_mma_kernel(const __grid_co
         for (int cb = cbeg; cb < cend; cb += 32) {
             const mma_block blk = mma_windows(p, box, elo, ehi, cb + lane, cend);
             const int nc = min(32, cend - cb);
-            if (__any_sync(0xffffffffu, !isfinite(blk.px + blk.py + blk.pz))) poison = NAN;
+            if (__any_sync(0xffffffffu, !isfinite(blk.px + blk.py + blk.pz))) {
+                poison = NAN;
+                spoiled = true;
+            }
             for (int j = 0; j < nc; j++) {
                 const int len = __shfl_sync(0xffffffffu, blk.len, j), k00 = __shfl_sync(0xffffffffu, blk.k0, j);
                 const int count = mma_count(len);
@@ -399,7 +404,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1) das_mma_kernel(const __grid_co
             if (since >= kMmaDrain) drain();
         }
     }
-    if (!fresh || drains == 0) drain();
+    // (a channel that spoils its voxels may have no window after the last drain)
+    if (!fresh || drains == 0 || spoiled) drain();
 
     if (warp >= 2 && __any_sync(0xffffffffu, odd) && lane == 0) *p.nonfinite = 1;
     // copies still in flight land before the CTA leaves

@@ -321,6 +321,34 @@ def test_tensor_core_batches(B, C, S, N, pitch):
         assert oracle.rel_l2(got.cpu().numpy(), ref) < TOL
 
 
+@pytest.mark.parametrize("V,C,S,late", [((128, 296), 260, 3, 0), ((40, 31), 260, 3, 0), ((128, 296), 260, 3, 40),
+                                        ((128, 296), 196, 1, 4)], ids=str)
+def test_tensor_core_batches_many_drains(V, C, S, late):
+    # up to 780 (channel, event) pairs per CTA, with (1240 voxels) and without (37888: a tile an SM)
+    # channel slices; `late`: the last channels lie outside the record, and no window
+    # follows the last drain
+    x, src, dst, offs, w = _problem(32, C, S, 256, *V, (0.5, 0.5), dtype=torch.float16, seed=late)
+    if late:
+        src[C - late:, 2] = 1e6
+    args = _dev(x, src, dst, offs, w)
+    got = ffdas_b200.das(*args)
+    info = _info()
+    assert info["variant"] == 10 and (info["kernels"] == 3) == (V != (40, 31))   # plan, products, fix-up: no slices
+    ref = _with_config({"variant": 1}, ffdas_b200.das, *args)
+    assert oracle.rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < TOL
+    cut = (slice(None), slice(None, None, 29), slice(None, None, 17))
+    few = _oracle(x, src, dst[cut[1:]].contiguous(), offs[cut].contiguous(), w[cut].contiguous())
+    assert oracle.rel_l2(got[:, ::29, ::17].cpu().numpy(), few) < TOL
+    if late:
+        # a NaN position among them has no window either, and the distance sqrt(1e-7)
+        # of the clamp: its taps reach every voxel through the fix-up
+        src[C - 1, 0] = float("nan")
+        args = _dev(x, src, dst, offs + 30.0, w)
+        got = ffdas_b200.das(*args)
+        ref = _with_config({"variant": 1}, ffdas_b200.das, *args)
+        assert oracle.rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < TOL
+
+
 def test_tensor_core_batches_channels_trailing_view_and_non_finite_values():
     # a (B, S, C, N) view; an infinite and a NaN sample, a NaN delay and an
     # infinite weight reach the values whose taps meet them and no others
