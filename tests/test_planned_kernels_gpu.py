@@ -349,6 +349,18 @@ def test_tensor_core_batches_many_drains(V, C, S, late):
         assert oracle.rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < TOL
 
 
+@pytest.mark.parametrize("C,S,N", [(48, 1, 512), (192, 9, 512), (100, 5, 1000)])
+def test_tensor_core_batches_are_no_less_exact_than_the_pair_kernels(C, S, N):
+    # 22-bit weights and truncated sums against FP32 weights and sums, on the same
+    # data, both against the oracle
+    x, src, dst, offs, w = _problem(32, C, S, N, 37, 59, (0.2 * N / 37, 0.5), dtype=torch.float16, seed=C)
+    args, ref = _dev(x, src, dst, offs, w), _oracle(x, src, dst, offs, w)
+    got = ffdas_b200.das(*args)
+    assert _info()["variant"] == 10
+    pairs = _with_config({"variant": 1}, ffdas_b200.das, *args)
+    assert oracle.rel_l2(got.cpu().numpy(), ref) <= oracle.rel_l2(pairs.cpu().numpy(), ref)
+
+
 def test_tensor_core_batches_channels_trailing_view_and_non_finite_values():
     # a (B, S, C, N) view; an infinite and a NaN sample, a NaN delay and an
     # infinite weight reach the values whose taps meet them and no others
