@@ -398,7 +398,7 @@ struct iq_bwd_layout {
 // window, four samples each with 128-bit shared accesses.  row(win, kw) gives
 // the window's gx row (null: nothing to add) and first sample.
 template <int WB, int REGION, int NW, class RowFn>
-__device__ __forceinline__ void iq_flush_bins(int *bins0, int lane, int warp, float finv, RowFn &&row) {
+__device__ __forceinline__ void iq_flush_bins(int *bins0, int lane, int warp, float finv, int n, RowFn &&row) {
     constexpr int GS = bin_stride(WB);
     constexpr int LPW = WB / 4, WPI = 32 / LPW;
     static_assert(WB % 4 == 0 && 32 % LPW == 0 && REGION % 4 == 0, "flush layout");
@@ -428,7 +428,9 @@ __device__ __forceinline__ void iq_flush_bins(int *bins0, int lane, int warp, fl
 #pragma unroll
             for (int i = 0; i < 4; i++)
                 if (s[0][i] | s[1][i]) atomicAdd(g + i, make_float2((float)s[0][i] * finv, (float)s[1][i] * finv));
-            if (last[0] | last[1]) atomicAdd(g + WB, make_float2((float)last[0] * finv, (float)last[1] * finv));
+            // (not past the row: see flush_bins)
+            if ((last[0] | last[1]) && kw + WB < n)
+                atomicAdd(g + WB, make_float2((float)last[0] * finv, (float)last[1] * finv));
         }
     }
 }
@@ -559,13 +561,13 @@ __global__ void __launch_bounds__(kStThreads, 2) das_iq_bwd_kernel(const iq_para
                         for (int j = 0; j < SC; j++) {
                             const uint32_t rr = mb[j] - k0p[j];
                             const bool in_rec = mb[j] - kFloorMagicBits < nlast;
-                            const bool staged = rr < (uint32_t)(WB - 1) && in_rec;
-                            const uint32_t at = staged ? groups + j * IG::group_bytes + rr * (uint32_t)IG::sample_bytes
-                                                       : zero_u32;
+                            const uint32_t at = rr < (uint32_t)(WB - 1) && in_rec
+                                                    ? groups + j * IG::group_bytes + rr * (uint32_t)IG::sample_bytes
+                                                    : zero_u32;
                             const bool ovfw = !FAST && k0p[j] == kOvf;
                             // a tap outside the record scatters zeros (into its window's
                             // bins, or the zero-only bin past the window)
-                            const float ws = staged ? w[j] * fscale : 0.f;
+                            const float ws = in_rec ? w[j] * fscale : 0.f;
                             const float wst = ws * t[j];
                             const uint32_t gb = gwin_u32 + (j * BT * 2 * GS + min(rr, (uint32_t)WB)) * 4;
                             float qj = 0.f, qx = 0.f;
@@ -638,12 +640,11 @@ __global__ void __launch_bounds__(kStThreads, 2) das_iq_bwd_kernel(const iq_para
                 consumer_sync();   // every consumer warp finished this stage's scatter
                 if (!dead) {
                     if (gx && fixed) {
-                        iq_flush_bins<WB, L::region, NW>(gstage, cx.lane, cx.warp, finv, [&](int win, int &kw) -> float2 * {
+                        iq_flush_bins<WB, L::region, NW>(gstage, cx.lane, cx.warp, finv, p.N, [&](int win, int &kw) -> float2 * {
                             const int grp = win / BT, b = win % BT;
                             const int cl = grp / SC, j = grp % SC;
                             kw = (int)(sm.meta[stage * kStWin + grp] - kFloorMagicBits);
-                            // (a window past the record, or read from the rows, has nothing in its bins)
-                            if (b0 + b >= p.B || c0 + cl >= cend || (unsigned)kw >= (unsigned)p.N) return nullptr;
+                            if (b0 + b >= p.B || c0 + cl >= cend) return nullptr;
                             return gx + (((int64_t)(b0 + b) * p.C + (c0 + cl)) * p.S + (e0 + j)) * p.N;
                         });
                     }

@@ -288,7 +288,7 @@ constexpr int bin_stride(int wb) { return (wb + 2 + 3) / 4 * 4; }
 // conflicts); the window's first lane also takes bin WB.  row(win, kw) returns
 // the gx row of the window (nullptr when it adds nothing) and its first sample.
 template <int WB, int REGION, class RowFn>
-__device__ __forceinline__ void flush_bins(int *bins0, int lane, int warp, float finv, RowFn &&row) {
+__device__ __forceinline__ void flush_bins(int *bins0, int lane, int warp, float finv, int n, RowFn &&row) {
     constexpr int GS4 = bin_stride(WB);
     constexpr int LPW = WB / 4;     // lanes per window
     constexpr int WPI = 32 / LPW;   // windows per warp and pass
@@ -317,7 +317,10 @@ __device__ __forceinline__ void flush_bins(int *bins0, int lane, int warp, float
             if (s1) atomicAdd(g + 1, (float)s1 * finv);
             if (s2) atomicAdd(g + 2, (float)s2 * finv);
             if (s3) atomicAdd(g + 3, (float)s3 * finv);
-            if (last) atomicAdd(g + WB, (float)last * finv);   // only q == 0 has one
+            // only q == 0 has one.  A tap in the record that misses its window (of a
+            // voxel without a finite position, which the tile's box leaves out) lands
+            // here too: not past the row, of which the window may be the end
+            if (last && kw + WB < n) atomicAdd(g + WB, (float)last * finv);
         }
     }
 }
@@ -2071,10 +2074,10 @@ __global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_kernel(const sta
                 if (!dead) {
                     // flush the stage's gradient slots: one red.add per touched sample
                     if (p.gx && fixed) {
-                        flush_bins<WB, kRegion>(gstage, cx.lane, cx.warp, finv, [&](int win, int &kw) -> float * {
+                        flush_bins<WB, kRegion>(gstage, cx.lane, cx.warp, finv, p.N, [&](int win, int &kw) -> float * {
                             const int cl = win / SC, j = win % SC;
                             kw = (int)(sm.meta[stage * kStWin + win] - kFloorMagicBits);
-                            if (c0 + cl >= cend || kw >= p.N) return nullptr;
+                            if (c0 + cl >= cend) return nullptr;
                             return p.gx + (((int64_t)cx.b * p.C + (c0 + cl)) * p.S + (e0 + j)) * p.N;
                         });
                     }
@@ -2443,11 +2446,11 @@ __global__ void __launch_bounds__(kStThreads, 2) das_staged_bwd_batch_kernel(con
                 consumer_sync();
                 if (!dead) {
                     if (p.gx && fixed) {
-                        flush_bins<WB, kRegion>(gstage, cx.lane, cx.warp, finv, [&](int win, int &kw) -> float * {
+                        flush_bins<WB, kRegion>(gstage, cx.lane, cx.warp, finv, p.N, [&](int win, int &kw) -> float * {
                             const int grp = win / BT, bi = win % BT;
                             const int cl = grp / SC, j = grp % SC;
                             kw = (int)(sm.meta[stage * kStWin + grp] - kFloorMagicBits);
-                            if (b0 + bi >= p.B || c0 + cl >= cend || kw >= p.N) return nullptr;
+                            if (b0 + bi >= p.B || c0 + cl >= cend) return nullptr;
                             return p.gx + (((int64_t)(b0 + bi) * p.C + (c0 + cl)) * p.S + (e0 + j)) * p.N;
                         });
                     }

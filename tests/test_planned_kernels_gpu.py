@@ -110,6 +110,39 @@ def test_calls_without_tensor_maps(B, beta):
     assert oracle.rel_l2(out.cpu().numpy(), ref + beta * old.numpy()) < TOL
 
 
+@pytest.mark.parametrize("dtype,B", [(torch.float32, 1), (torch.float32, 3), (torch.complex64, 2)], ids=str)
+def test_adjoint_of_a_voxel_without_a_position_stays_in_its_rows(dtype, B):
+    # a NaN position has the distance sqrt(1e-7) of the clamp and no part in its tile's
+    # window: a tap in the record, but 60 samples before the window, at the record's end
+    C, S, N = 9, 4, 300
+    x, src, dst, offs, w = _problem(B, C, S, N, 64, 40, (0.05, 0.05), dtype=dtype, z0=60.0)
+    offs = offs - offs.mean() + (N - 80.0)
+    clean = offs.clone()
+    dst[30, 20] = float("nan")
+    args = [t.contiguous() for t in _dev(x, src, dst, offs, w)]
+    cplx = dtype.is_complex
+    gout = torch.ones((B, 64, 40), device=DEV, dtype=dtype)
+    room = torch.zeros(B * C * S * N + 4096, device=DEV, dtype=dtype)      # the gradient, and what follows it
+    L, h = _lib.load(), ffdas_b200.get_library_handle(torch.device(DEV))
+    h.set_stream(torch.cuda.current_stream().cuda_stream)
+    dt = _lib.DataType.C_32F if cplx else _lib.DataType.R_32F
+    xd, gd = _lib.TensorDesc(list(x.shape), None, dt), _lib.TensorDesc(list(gout.shape), None, dt)
+    p = [t.data_ptr() for t in args]
+    _lib.check(L.ffdas_das_backward(h.h, p[1], None, 0.0, xd.desc, p[0], p[2], p[3], p[4], 0, None, gd.desc, gout.data_ptr(),
+                                    room.data_ptr(), None, None, None, None))
+    assert _info()["variant"] == (8 if cplx else 4)
+    assert (room[B * C * S * N:] == 0).all()
+    gx = room[: B * C * S * N].reshape(x.shape)
+    # every other voxel's taps, as without it
+    w2 = w.clone()
+    w2[:, 30, 20] = 0.0
+    dst[30, 20] = dst[30, 21]
+    xr = x.to(torch.complex128 if cplx else torch.float64).requires_grad_(True)
+    das_ref(xr, *(t.double() for t in (src, dst, clean, w2))).sum().real.backward()
+    few = (gx.cpu() - xr.grad).abs()
+    assert few[..., N - 60:].norm() < TOL * xr.grad.norm()
+
+
 def _with_config(config, f, *args, **kw):
     h = ffdas_b200.get_library_handle(torch.device(DEV))
     h.set_config(config)
