@@ -248,8 +248,11 @@ __global__ void __launch_bounds__(kMmaThreads, 1) das_mma_kernel(const __grid_co
     }
     for (int e = threadIdx.x; e < p.S; e += kMmaThreads) {
         const int lo = ilo[e], hi = ihi[e];
-        olo[e] = lo == INT_MAX ? INFINITY : unordered(lo);     // no finite delay: no window
-        ohi[e] = hi == INT_MIN ? -INFINITY : unordered(hi);
+        float flo = lo == INT_MAX ? INFINITY : unordered(lo);     // no finite delay: no window
+        float fhi = hi == INT_MIN ? -INFINITY : unordered(hi);
+        widen_delays(flo, fhi);
+        olo[e] = flo;
+        ohi[e] = fhi;
     }
     gram_tc::fence_before_sync();
     __syncthreads();

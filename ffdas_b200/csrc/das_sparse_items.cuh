@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(kStThreads, 2) das_sparse_items_kernel(const s
                         lo = fminf(lo, sm.red[(ww * 16 + cx.tid) * 2]);
                         hi = fmaxf(hi, sm.red[(ww * 16 + cx.tid) * 2 + 1]);
                     }
+                    widen_delays(lo, hi);
                     sm.ofs_lo[cx.tid] = lo;
                     sm.ofs_hi[cx.tid] = hi;
                 }

@@ -254,14 +254,18 @@ constexpr float kSaneRange = 1048576.0f;   // 2^20: tau, offsets and distances b
 // millions of samples away) meet the record all the same, and their windows
 // grow with that rounding; without it an in-record tap missed its window (left
 // out of the image, and in the adjoints added past its window's bins).
+// The delays' share is added to olo and ohi once a pass (widen_delays), that of
+// the distances here.
+constexpr float kFarRounding = 2e-6f;
+__device__ __forceinline__ void widen_delays(float &olo, float &ohi) {
+    if (!(olo <= ohi)) return;   // no finite delay in the tile: inf, -inf
+    const float m = kFarRounding * fmaxf(fabsf(olo), fabsf(ohi));
+    olo -= m;
+    ohi += m;
+}
 __device__ __forceinline__ void tap_range(float olo, float ohi, float rmin, float rmax, float &lo, float &hi) {
-    lo = floorf(olo + rmin) - 2.f;
-    hi = floorf(ohi + rmax) + 2.f;
-    const float far = fmaxf(fabsf(olo), fabsf(ohi)) + rmax;
-    if (far > kSaneRange) {   // (no finite delay in the tile: lo = inf and hi = -inf stay)
-        if (lo <= 3e38f) lo -= 2e-6f * far;
-        if (hi >= -3e38f) hi += 2e-6f * far;
-    }
+    lo = floorf(olo + __fmaf_rn(rmax, -kFarRounding, rmin)) - 2.f;
+    hi = floorf(__fmaf_rn(rmax, 1.f + kFarRounding, ohi)) + 2.f;
 }
 
 template <int WB, int K>
@@ -587,6 +591,7 @@ __device__ __forceinline__ void staged_pass_begin(const staged_params &p, staged
                 lo = fminf(lo, sm.red[(ww * 16 + cx.tid) * 2]);
                 hi = fmaxf(hi, sm.red[(ww * 16 + cx.tid) * 2 + 1]);
             }
+            widen_delays(lo, hi);
             sm.ofs_lo[cx.tid] = lo;
             sm.ofs_hi[cx.tid] = hi;
         }
@@ -771,6 +776,7 @@ __device__ __forceinline__ void staged_pass_begin2(const staged_params &p, stage
                 lo = fminf(lo, sm.red[(ww * 16 + cx.tid) * 2]);
                 hi = fmaxf(hi, sm.red[(ww * 16 + cx.tid) * 2 + 1]);
             }
+            widen_delays(lo, hi);
             sm.ofs_lo[cx.tid] = lo;
             sm.ofs_hi[cx.tid] = hi;
         }

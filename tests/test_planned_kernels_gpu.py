@@ -430,6 +430,102 @@ def test_pair_buffer_only_where_the_backward_reads_it(kind, variant, kept):
     assert torch.isfinite(offs.grad).all() and offs.grad.abs().max() > 0
 
 
+_CAPTURED = dict(staged=(1, 1200, 4, torch.float32, 2), batch=(3, 200, 3, torch.float32, 2), products=(33, 40, 3, torch.float16, 10),
+                 iq=(3, 20, 4, torch.complex64, 2), iq_copied=(1, 20, 1, torch.complex64, 2), entries=(4, 1000, 4, torch.float32, 9))
+
+
+@pytest.mark.parametrize("kind", _CAPTURED)
+def test_captured_call_follows_its_inputs(kind):
+    # a graph of one unscheduled call: the plan, its overlapped ingest, both widths,
+    # the sort, the clearing of sliced images -- all made again at each replay, for
+    # new data and for delays of another spread
+    B, C, S, dtype, variant = _CAPTURED[kind]
+    N = 501 if kind == "iq_copied" else 512
+    x, src, dst, offs, w = _problem(B, C, S, N, 131, 67, (0.4, 0.5), dtype=dtype)
+    args = _dev(x, src, dst, offs, w)
+    if kind == "entries":
+        idx = _lists(S, S, (131, 67), seed=1)[0].to(DEV)
+        call = lambda out=None: ffdas_b200.das_sparse(*args, idx, out=out)  # noqa: E731
+    else:
+        call = lambda out=None: ffdas_b200.das(*args, out=out)  # noqa: E731
+    out = call()
+    assert _info()["variant"] == variant
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        call(out)
+    for spread in (1.0, 1.9):
+        args[0].copy_(args[0].roll(7, dims=-1))
+        args[3].copy_(offs.to(DEV) * spread)
+        ref = call()
+        out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        # the same taps; sums that meet in atomics come in another order
+        assert oracle.rel_l2(out.cpu().numpy(), ref.cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("per_item", [False, True])
+def test_channel_scale_and_beta_on_the_iq_and_entry_kernels(per_item):
+    L, h = _lib.load(), ffdas_b200.get_library_handle(torch.device(DEV))
+    for kind in ("iq", "entries"):
+        B, C, S, dtype = (2, 24, 4, torch.complex64) if kind == "iq" else (4, 1000, 4, torch.float32)
+        x, src, dst, offs, w = _problem(B, C, S, 300, 131, 67, dtype=dtype)
+        idx = _lists(S, S, (131, 67), seed=1)[0] if kind == "entries" else None
+        g = torch.rand((B, C) if per_item else (C,), generator=torch.Generator().manual_seed(3)) + 0.5
+        args = _dev(x, src, dst, offs, w)
+        call = (lambda *a, **k: ffdas_b200.das_sparse(*a, idx.to(DEV), **k)) if kind == "entries" else ffdas_b200.das
+        got = call(*args, channel_scale=g.to(DEV))
+        assert _info()["variant"] == (2 if kind == "iq" else 9)
+        xs = x * g.reshape(-1, C, 1, 1)
+        ref = _with_config({"variant": 1}, call, xs.to(DEV), *args[1:])
+        assert oracle.rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < TOL
+        # beta through the C entry: out = beta * out + image, with and without channel slices
+        old = torch.randn(got.shape, generator=torch.Generator().manual_seed(4), dtype=got.dtype)
+        out, plain = old.to(DEV), call(*args)
+        beta = (ctypes.c_float * 2)(0.5, 0.25 if kind == "iq" else 0.0)
+        h.set_stream(torch.cuda.current_stream().cuda_stream)
+        dt = _lib.DataType.C_32F if kind == "iq" else _lib.DataType.R_32F
+        xd, od = _lib.TensorDesc(list(x.shape), None, dt), _lib.TensorDesc(list(out.shape), None, dt)
+        p, b = [t.data_ptr() for t in args], ctypes.cast(beta, ctypes.c_void_p)
+        if kind == "iq":
+            _lib.check(L.ffdas_das(h.h, p[1], None, 0.0, xd.desc, p[0], p[2], p[3], p[4], b, od.desc, out.data_ptr(), 0, 0))
+        else:
+            i = idx.to(DEV)
+            _lib.check(L.ffdas_das_sparse(h.h, p[1], None, 0.0, xd.desc, p[0], p[2], p[3], p[4], S, i.data_ptr(), b, od.desc,
+                                          out.data_ptr(), 0, 0))
+        assert _info()["variant"] == (2 if kind == "iq" else 9)
+        want = plain.cpu() + (complex(0.5, 0.25) if kind == "iq" else 0.5) * old
+        assert oracle.rel_l2(out.cpu().numpy(), want.numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex32])
+@pytest.mark.parametrize("need", ["x", "weights", "offsets", "srcpos", "dstpos", "dstpos,offsets", "x,weights"])
+def test_iq_adjoint_subsets(dtype, need):
+    # each gradient by itself (the kernel scatters, sums and clears only what is asked
+    # for) against all of them at once; complex32 data at odd sizes
+    x, src, dst, offs, w = _problem(3, 21, 5, 301, 24, 19, (1.1, 0.6), dtype=torch.complex64, seed=9)
+    x = x.to(dtype)
+    names = ("x", "srcpos", "dstpos", "offsets", "weights")
+    gy = torch.randn((3, 24, 19), generator=torch.Generator().manual_seed(1), dtype=torch.complex64).to(DEV)
+    some, every = ([t.to(DEV).requires_grad_(n in which) for n, t in zip(names, (x, src, dst, offs, w))]
+                   for which in (need.split(","), names))
+    for leaf in (some, every):
+        ffdas_b200.das(*leaf, wavenum=0.4).backward(gy)
+        assert _info()["variant"] == 8
+    for n, a, b in zip(names, some, every):
+        if n in need.split(","):
+            # fixed-point sums are exact in any order; the rest differ by the order of FP32 sums
+            assert oracle.rel_l2(a.grad.cfloat().cpu().numpy(), b.grad.cfloat().cpu().numpy()) < 1e-5
+    if dtype == torch.complex32:   # the same numbers in single precision
+        ref = [t.detach().cfloat() if t.is_complex() else t.detach() for t in every]
+        ref = [t.clone().requires_grad_(True) for t in ref]
+        ffdas_b200.das(*ref, wavenum=0.4).backward(gy)
+        for n, a, b in zip(names, every, ref):   # (x's gradient comes back in 11 bits)
+            assert oracle.rel_l2(a.grad.cfloat().cpu().numpy(), b.grad.cfloat().cpu().numpy()) < (1e-3 if n == "x" else TOL)
+
+
 @pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9, 16, 17, 31, 32])
 @pytest.mark.parametrize("S", [33, 97])
 def test_select_sizes(k, S):

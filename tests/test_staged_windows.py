@@ -211,18 +211,17 @@ def test_fast_path_plane_wave_frame():
 
 
 # ---------------------------------------------------------------------------
-# Far distances cancelled by far delays (tap_range in csrc/das_staged.cuh)
+# Far distances cancelled by far delays (widen_delays, tap_range in csrc/das_staged.cuh)
 
 F = np.float32
 
 
 def tap_range(olo, ohi, rmin, rmax, grow=True):
-    lo = np.floor(F(olo + rmin)) - F(2)
-    hi = np.floor(F(ohi + rmax)) + F(2)
-    far = F(max(abs(olo), abs(ohi)) + rmax)
-    if grow and far > SANE:
-        lo, hi = F(lo - F(2e-6) * far), F(hi + F(2e-6) * far)
-    return lo, hi
+    if grow:                                   # widen_delays, and the distances' share (fused: one rounding)
+        m = F(F(2e-6) * max(abs(olo), abs(ohi)))
+        olo, ohi = F(olo - m), F(ohi + m)
+        rmin, rmax = F(np.float64(rmin) - np.float64(F(2e-6)) * rmax), np.float64(rmax) * np.float64(F(1) + F(2e-6))
+    return np.floor(F(olo + rmin)) - F(2), np.floor(F(ohi + rmax)) + F(2)
 
 
 def far_tile(far, seed=0):
