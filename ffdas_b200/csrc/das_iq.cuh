@@ -196,11 +196,12 @@ __device__ __forceinline__ void iq_event_phases(const iq_params &q, bool active,
         E[j] = (active && j < sc) ? iq_phase(ofs[j], q.turn_hi, q.turn_lo) : make_float2(0.f, 0.f);
 }
 
-// apply_directivity; an excluded channel has no factor either: one infinitely far
-// away (its distance and factor are NaN) is excluded too, and adds nothing.
-__device__ __forceinline__ void iq_directivity(recv_geom &g, float2 &R, const staged_ctx &cx, float4 c, float4 dir) {
-    apply_directivity(g, cx.vx, cx.vy, cx.vz, c.x, c.y, c.z, dir);
-    if (g.rsq == 1e30f) R = make_float2(0.f, 0.f);
+// Distance whose phase is a channel's factor.  With directivity a channel
+// infinitely far away (its distance is NaN) lies outside every cone and adds
+// nothing: it keeps a finite factor.
+__device__ __forceinline__ float iq_distance(const recv_geom &g, const float4 *srcdir) {
+    const float r = g.rsq * g.rinv;
+    return srcdir ? fminf(r, 1e30f) : r;
 }
 
 // Floor split of the delays of two events of a channel (SC >= 2), or one.
@@ -285,8 +286,10 @@ __global__ void __launch_bounds__(kStThreads, 3) das_iq_kernel(const iq_params q
                         const int c = c0 + cl;
                         const float4 cp = sm.chan_pos[stage * kStWin + cl];
                         recv_geom g = receive_geometry(cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z);
-                        float2 R = iq_phase(g.rsq * g.rinv, q.turn_hi, q.turn_lo);
-                        if (p.srcdir) iq_directivity(g, R, cx, cp, sm.chan_dir[stage * kStWin + cl]);
+                        const float2 R = iq_phase(iq_distance(g, p.srcdir), q.turn_hi, q.turn_lo);
+                        if (p.srcdir)
+                            apply_directivity(g, cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z,
+                                              sm.chan_dir[stage * kStWin + cl]);
                         uint32_t k0p[SC], mb[SC];
                         float t[SC];
                         load_meta<SC>(sm.meta, stage, cl, k0p);
@@ -544,8 +547,10 @@ __global__ void __launch_bounds__(kStThreads, 2) das_iq_bwd_kernel(const iq_para
                         const int c = c0 + cl;
                         const float4 cp = sm.chan_pos[stage * kStWin + cl];
                         recv_geom gm = receive_geometry(cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z);
-                        float2 R = iq_phase(gm.rsq * gm.rinv, qp.turn_hi, qp.turn_lo);
-                        if (p.srcdir) iq_directivity(gm, R, cx, cp, sm.chan_dir[stage * kStWin + cl]);
+                        const float2 R = iq_phase(iq_distance(gm, p.srcdir), qp.turn_hi, qp.turn_lo);
+                        if (p.srcdir)
+                            apply_directivity(gm, cx.vx, cx.vy, cx.vz, cp.x, cp.y, cp.z,
+                                              sm.chan_dir[stage * kStWin + cl]);
                         float2 h[BT];
 #pragma unroll
                         for (int b = 0; b < BT; b++)
