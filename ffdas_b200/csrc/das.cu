@@ -724,12 +724,13 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
 
     // Complex (IQ) data on the staged complex kernel when the schedule asks
     // for variant 2: 256-voxel tiles, the gather kernel's event chunk so that
-    // both sum in the same order.  The planner keeps complex data on the
-    // gather kernel: measured on B200 the two are level for single frames
-    // (3-D diverging volume, 1024 channels: 146 ms staged, 152 ms gather,
-    // 284 ms reference ALG1) -- both bound by the per-tap sincos and complex
-    // multiply-add -- and the gather kernel's batch tiles share the phase
-    // over frames (50-frame ensemble: 9.9 ms gather, 34.6 ms staged).
+    // both sum in the same order.  (Without a schedule dense complex data took
+    // the IQ batch tiles above.)  Measured on B200 it is level with the gather
+    // kernel for single frames (3-D diverging volume, 1024 channels: 146 ms
+    // staged, 152 ms gather, 284 ms reference ALG1) -- both bound by the
+    // per-tap sincos and complex multiply-add -- and slower for batches, whose
+    // gather tiles share the phase over frames (50 frames: 9.9 ms gather, 34.6
+    // ms staged).
     if ((kind == ST_C32 || kind == ST_C16) && od.dtype == FFDAS_C_32F && !a.sparse && staged_batch_supported() &&
         npad >= 64 && rows < INT32_MAX && pb.B <= 65535 && h.has_config && h.config.variant == 2) {
         gather_params cg = gp;
@@ -782,6 +783,10 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
             SC = full && work <= 2 * (int64_t)std::max(h.sm_count, 1) ? 8 : 4;
         }
         h.last.variant = 2;
+        if (plan) {   // the shape is the device's choice: the voxels of a tile
+            h.last.tile_x = plan_tile;
+            h.last.tile_y = h.last.tile_z = 1;
+        }
         h.last.batch_tile = s.BT;
         h.last.event_chunk = SC;
         h.last.grid = tiles * bchunks_st * csplit;

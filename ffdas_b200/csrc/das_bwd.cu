@@ -945,8 +945,12 @@ ffdas_error_t das_backward(ffdas_context &h, const das_call &a, const ffdas_tens
         h.last = ffdas_kernel_info_t{};
         h.last.variant = 4;
         h.last.tile_x = bp.T0; h.last.tile_y = bp.T1; h.last.tile_z = bp.T2;
+        if (plan) {   // the shape is the device's choice: the voxels of a tile
+            h.last.tile_x = 256;
+            h.last.tile_y = h.last.tile_z = 1;
+        }
         h.last.batch_tile = BT; h.last.event_chunk = SC; h.last.storage = kind;
-        // (ingest,) adjoint; the plan and the width not taken are not counted
+        // (ingest,) adjoint; the plan, the clearing and the width not taken are not counted
         h.last.kernels = h.last_pairs_reused ? 1 : 2;
         h.last.grid = stiles * bchunks_st * csplit;
         if (bchunks_st > 65535) return FFDAS_ERROR_DIMS_TOO_LARGE;

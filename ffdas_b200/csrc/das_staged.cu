@@ -62,7 +62,7 @@ static int staged_pair_bytes(int kind) {
 // 2-D map over the pair rows (one row per item, channel, event); a 16-byte
 // (complex f32) pair is two 8-byte elements, so its x coordinates and box
 // width count elements, not pairs.
-ffdas_error_t pair_row_map(CUtensorMap &map, const void *P, int64_t npad, int64_t rows, int kind, int WB) {
+static ffdas_error_t pair_row_map(CUtensorMap &map, const void *P, int64_t npad, int64_t rows, int kind, int WB) {
     auto encode = tensor_map_encoder();
     if (!encode) return FFDAS_ERROR_CUDA_DRIVER;
     const int pair_bytes = staged_pair_bytes(kind);
@@ -79,18 +79,17 @@ ffdas_error_t pair_row_map(CUtensorMap &map, const void *P, int64_t npad, int64_
 }
 
 // 3-D map over the same rows for batch tiles: dims {npad, C*S, B}, box
-// {WB, 1, BT}; batch items past B read as zeros.  16-byte pairs as above.
-ffdas_error_t pair_batch_map(CUtensorMap &map, const void *P, int64_t npad, int64_t cs, int64_t B, int kind,
+// {WB, 1, BT}; batch items past B read as zeros.
+static ffdas_error_t pair_batch_map(CUtensorMap &map, const void *P, int64_t npad, int64_t cs, int64_t B, int kind,
                                     int WB, int BT) {
     auto encode = tensor_map_encoder();
     if (!encode) return FFDAS_ERROR_CUDA_DRIVER;
-    const int pair_bytes = staged_pair_bytes(kind);
-    const int units = pair_bytes == 16 ? 2 : 1;
-    const cuuint64_t dims[3] = {(cuuint64_t)(npad * units), (cuuint64_t)cs, (cuuint64_t)B};
+    const int pair_bytes = (kind == ST_F32) ? 8 : 4;
+    const cuuint64_t dims[3] = {(cuuint64_t)npad, (cuuint64_t)cs, (cuuint64_t)B};
     const cuuint64_t strides[2] = {(cuuint64_t)npad * pair_bytes, (cuuint64_t)(cs * npad * pair_bytes)};
-    const cuuint32_t box[3] = {(cuuint32_t)(WB * units), 1u, (cuuint32_t)BT};
+    const cuuint32_t box[3] = {(cuuint32_t)WB, 1u, (cuuint32_t)BT};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
-    const CUresult r = encode(&map, pair_bytes >= 8 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32,
+    const CUresult r = encode(&map, pair_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32,
                               3, const_cast<void *>(P), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

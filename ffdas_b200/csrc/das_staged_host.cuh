@@ -55,9 +55,6 @@ inline int balanced_slices(int64_t ctas, int sms, int resident, int most) {
 }
 
 // Defined in das_staged.cu.
-ffdas_error_t pair_batch_map(CUtensorMap &map, const void *P, int64_t npad, int64_t cs, int64_t B, int kind, int WB,
-                             int BT);
-ffdas_error_t pair_row_map(CUtensorMap &map, const void *P, int64_t npad, int64_t rows, int kind, int WB);
 staged_params base_params(ffdas_context &h, const das_problem &pb, const gather_params &gp);
 
 }  // namespace ffdas

@@ -12,6 +12,12 @@ input (or takes it in place with `run.replay()` after writing `run.x`),
 replays the graph, and returns the static output (overwritten by the next
 call unless `clone=True`).  Geometry tensors must not change after capture
 (their device addresses are baked into the graph).
+
+The schedule a runner (or a DASStream) works with stays set on the device's
+library handle, so that plain calls afterwards compute as it does; with one set
+they take the kernels it names and not those that plan tiles for themselves, the
+IQ, tensor-core and sorted-list ones among them.
+`get_library_handle(device).set_config(None)` returns to the planner's choice.
 """
 from __future__ import annotations
 

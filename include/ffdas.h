@@ -174,6 +174,14 @@ typedef struct {
 } ffdas_das_config_t;
 
 /* What the last das/das_sparse/backward call on a handle launched (new).
+ * variant of a forward: 1 gather, 2 TMA-staged (real data, or complex data on
+ * batch tiles), 5 direct, 6 das_sparse over bucketed lists, 9 das_sparse over
+ * sorted entries, 10 half-precision batches on the tensor cores; of an adjoint:
+ * see ffdas_das_backward.  A call without a schedule chooses the tile shape
+ * and window width of the staged kernels on the device: tile_x then holds the
+ * voxels of a tile (tile_y = tile_z = 1), event_chunk that of the 32-sample
+ * windows, and grid counts the CTAs of the largest shape, of which those past
+ * the chosen one return at once.
  * After ffdas_truncate_rank, variant is its eigen route: 10 orthogonal
  * iteration on the device, 11 cuSOLVER syevd, 12 syevdx over one index
  * range, 13 keep-all copy; grid is the Gram kernel's CTA count and
@@ -184,7 +192,8 @@ typedef struct {
     int32_t batch_tile;
     int32_t event_chunk;
     int32_t storage;      /* pair storage: 0 f32, 1 f16, 2 bf16, 3 f64, 4 c32, 5 c16, 6 c64 */
-    int32_t kernels;      /* kernels launched by the call */
+    int32_t kernels;      /* kernels launched by the call (ffdas_das_backward on real data: the ingest,
+                             if any, and the adjoint) */
     int64_t grid;         /* CTAs of the main kernel */
     int32_t copy_engine;  /* staged kernels: 1 TMA, 2 cp.async; 0 otherwise */
 } ffdas_kernel_info_t;
@@ -237,7 +246,11 @@ FFDAS_API ffdas_error_t ffdas_contiguous_copy(
  * out[b, v] = beta * out[b, v] + sum_s sum_c w[s,v] * lerp(x[b,c,s,:], tau)
  * with tau = offsets[s,v] + |dstpos[v] - srcpos[c]|.
  * offsets/weights are indexed [s * V + v] for both 3-D and 4-D x (the
- * reference reuses event 0's row for 3-D x; see the design notes). */
+ * reference reuses event 0's row for 3-D x; see the design notes).
+ * The same call gives the same bits again unless its sums meet in atomics:
+ * grids too small to fill the GPU split the channels into slices that add into
+ * the image, and das_sparse on long lists adds a voxel's entries as they come.
+ * Those images differ from call to call by the rounding of FP32 sums. */
 FFDAS_API ffdas_error_t ffdas_das(
     ffdas_handle_t handle,
     const float *srcpos,
@@ -298,7 +311,11 @@ FFDAS_API ffdas_error_t ffdas_das_sparse(
  * dense calls), 3 (gather adjoint: dense calls under schedule variant 3 or
  * with directivity, and das_sparse under variant 3 or when the lists' tables
  * do not fit), 7 (das_sparse: a lane per list entry, entries bucketed by
- * event) or 8 (complex data: a thread per voxel). */
+ * event) or 8 (complex data: dense calls without a schedule on staged batch
+ * tiles, others a thread per voxel).  Sums that meet in atomics (the gradients
+ * of x and of the channel positions, and those of voxels shared by several
+ * items or channel slices) come in any order; grad_x of dense calls is summed in
+ * steps of 2^-22 of the largest |grad_out| |weight| of a tile and event chunk. */
 FFDAS_API ffdas_error_t ffdas_das_backward(
     ffdas_handle_t handle,
     const float *srcpos,
