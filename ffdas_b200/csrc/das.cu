@@ -142,7 +142,8 @@ static size_t storage_bytes(int kind) {
 // ---------------------------------------------------------------- ingest ---
 template <typename Tin, int K>
 static ffdas_error_t launch_ingest_t(ffdas_context &h, const das_problem &pb, const void *x,
-                                     int64_t npad, void *P, const float *gain, int gain_bstride, bool beside_plan) {
+                                     int64_t npad, void *P, const float *gain, int gain_bstride, bool beside_plan,
+                                     const int *skip) {
     const int64_t rows = (int64_t)pb.B * pb.C * pb.S;
     if (rows == 0) return FFDAS_SUCCESS;
     const int64_t bc = (int64_t)pb.B * pb.C;
@@ -150,6 +151,8 @@ static ffdas_error_t launch_ingest_t(ffdas_context &h, const das_problem &pb, co
     const int64_t per_block = (int64_t)kIngestThreads * kIngestVec;
     dim3 grid((unsigned)((npad + per_block - 1) / per_block), (unsigned)std::min<int64_t>(pb.S, 65535),
               (unsigned)std::min<int64_t>(bc, 65535));
+    // blocks that may have nothing to do are few, and walk the rows
+    if (skip) grid.z = std::min(grid.z, std::max(1u, 4096u / (grid.x * grid.y)));
     cudaLaunchAttribute overlap;
     overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     overlap.val.programmaticStreamSerializationAllowed = 1;
@@ -162,7 +165,7 @@ static ffdas_error_t launch_ingest_t(ffdas_context &h, const das_problem &pb, co
     lc.numAttrs = beside_plan ? 1 : 0;
     FFDAS_CUDA(cudaLaunchKernelEx(&lc, ingest_pairs_kernel<Tin, K>, static_cast<const Tin *>(x), pb.x_bstride, pb.x_cstride,
                                   pb.x_sstride, pb.C, pb.S, pb.N, (int)bc, npad,
-                                  static_cast<typename pair_traits<K>::storage *>(P), gain, gain_bstride));
+                                  static_cast<typename pair_traits<K>::storage *>(P), gain, gain_bstride, skip));
     return ffdas_launch_check(h.stream);
 }
 
@@ -185,12 +188,14 @@ static ffdas_error_t channel_gain(const ffdas_context &h, const das_problem &pb,
 }
 
 // beside_plan: the launch before is the call's tile plan, which this one overlaps.
+// skip: device word, nonzero when nothing reads the pairs (not beside the plan).
 static ffdas_error_t launch_ingest(ffdas_context &h, const das_problem &pb, ffdas_datatype_t xt,
-                                   int kind, const void *x, int64_t npad, void *P, bool beside_plan = false) {
+                                   int kind, const void *x, int64_t npad, void *P, bool beside_plan = false,
+                                   const int *skip = nullptr) {
     const float *gain = nullptr;
     int gain_bstride = 0;
     FFDAS_TRY(channel_gain(h, pb, &gain, &gain_bstride));
-#define FFDAS_INGEST(Tin, K) launch_ingest_t<Tin, K>(h, pb, x, npad, P, gain, gain_bstride, beside_plan)
+#define FFDAS_INGEST(Tin, K) launch_ingest_t<Tin, K>(h, pb, x, npad, P, gain, gain_bstride, beside_plan, skip)
     switch (xt) {
         case FFDAS_R_32F:
             if (kind == ST_F32) return FFDAS_INGEST(float, ST_F32);
@@ -580,8 +585,11 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
                              asked ? h.config.tile_x : 0);
     }
 
-    // ---- large half-precision batches: tensor cores, straight from x ----
-    if (way == route::mma) return launch_mma(h, pb, a, static_cast<float *>(a.out));
+    // ---- large half-precision batches: tensor cores, straight from x; where the
+    // batch tiles can be faster (products_above) both are launched below and the
+    // plan of the batch tiles decides which of them runs ----
+    const bool contested = way == route::mma && mma_products_above(pb) >= 1.f;
+    if (way == route::mma && !contested) return launch_mma(h, pb, a, static_cast<float *>(a.out));
 
     // ---- dense complex (IQ) data without a schedule: batch tiles on windows of
     // plain samples (das_iq.cuh).  (A pair buffer stays unfilled: the adjoint of
@@ -644,6 +652,10 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     void *Pbase = nullptr;
     if (h.pair_buf && h.pair_buf_bytes >= pair_bytes + 256) {
         Pbase = h.pair_buf;
+    } else if (contested && P.alloc(pair_bytes + 256) != FFDAS_SUCCESS) {
+        return launch_mma(h, pb, a, static_cast<float *>(a.out));   // no room for pairs: none needed
+    } else if (contested) {
+        Pbase = P.get<void>();
     } else {
         FFDAS_TRY(P.alloc(pair_bytes + 256));   // after the pairs: das_sparse's gate word, the tile plan
         Pbase = P.get<void>();
@@ -658,11 +670,21 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     const int plan_tile = planned ? s.T0 * s.T1 * s.T2 : 0;
     const int64_t plan_tiles = plan_tile && pb.C > 0 ? plan_max_tiles(pb, plan_tile) : 0;
     void *const plan = plan_tiles > 0 && plan_tiles <= INT32_MAX ? static_cast<char *>(Pbase) + pair_bytes + 64 : nullptr;
+    if (contested && (!plan || s.BT == 1)) return launch_mma(h, pb, a, static_cast<float *>(a.out));
+    const int *products = nullptr;   // device word: the products run, not the batch tiles
     if (plan) {
-        const plan_params own = make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, npad, plan_tile,
+        plan_params own = make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, npad, plan_tile,
                                           s.BT > 1 ? kPlanBatch : kPlanForward, plan);
+        if (contested) {
+            own.products_above = mma_products_above(pb);
+            products = &static_cast<const tile_plan *>(plan)->products;
+            void *const mplan = static_cast<char *>(Pbase) + pair_bytes + 128;
+            const plan_params other =
+                make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, pb.N, kMmaTileVoxels, kPlanMma, mplan);
+            FFDAS_TRY(launch_tile_plan(h, own, &other));
+            FFDAS_TRY(launch_mma(h, pb, a, static_cast<float *>(a.out), mplan, products));
         // pair rows kept for a backward: the adjoint's plan beside the forward's
-        if (Pbase == h.pair_buf && plan_max_tiles(pb, 256) > 0) {
+        } else if (Pbase == h.pair_buf && plan_max_tiles(pb, 256) > 0) {
             const plan_params adjoint = make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, npad, 256, kPlanAdjoint,
                                                   static_cast<char *>(Pbase) + pair_bytes + 128);
             FFDAS_TRY(launch_tile_plan(h, own, &adjoint));
@@ -672,7 +694,7 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
             FFDAS_TRY(launch_tile_plan(h, own));
         }
     }
-    FFDAS_TRY(launch_ingest(h, pb, xd.dtype, kind, a.x, npad, Pbase, plan != nullptr));
+    FFDAS_TRY(launch_ingest(h, pb, xd.dtype, kind, a.x, npad, Pbase, plan && !contested, products));
     if (Pbase == h.pair_buf) {
         h.pair_sig.buf = h.pair_buf;
         h.pair_sig.x = a.x;
@@ -793,7 +815,12 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         // (plan,) ingest, (image preparation,) delay-and-sum, (the width not taken)
         h.last.kernels = (csplit > 1 ? 3 : 2) + (gp.plan ? (s.BT == 1 ? 2 : 1) : 0);
         if (bchunks_st > 65535) return FFDAS_ERROR_DIMS_TOO_LARGE;
-        h.mark_start();
+        if (contested) {   // the batch tiles, or what the products launched
+            h.last.variant = 10;
+            h.last.kernels += 2;
+        } else {
+            h.mark_start();
+        }
         const ffdas_error_t err = launch_staged(h, pb, kind, gp, SC, SC_wide, s.WB, s.BT, s.copy,
                                                 dim3((unsigned)tiles, (unsigned)bchunks_st, (unsigned)csplit));
         h.mark_stop();

@@ -19,6 +19,20 @@ bool mma_supported(const das_problem &pb, ffdas_datatype_t xt, ffdas_datatype_t 
            plan_max_tiles(pb, kMmaTile) > 0 && plan_max_tiles(pb, kMmaTile) <= INT32_MAX;
 }
 
+// A (channel, event) of a tile takes the products 1.3 us on an SM whatever the items;
+// the batch tiles take 0.45 ps a voxel and item of every event place, in passes of
+// four.  Where the windows fit they meet at 85 to 125 items of whole passes (times of
+// both, us: 160 channels, 3 events, 400 x 256 pixels, 32 items 1670 and 756; 92, 6,
+// 150 x 200, 64: 685 and 672; 192, 9, 299 x 102, 81: 2726 and 2572; 64, 3, 400 x 256,
+// 81: 661 and 809; 128, 8, 200 x 100, 128: 993 and 1265), and windows that overflow cost
+// the batch tiles up to 5.4 times that (192, 8, 100 x 64, 56: 953 and 2780).  Both are
+// launched below 100: what the loser costs, 12 us on a call of 300 and 20 on one of 100,
+// buys the choice.
+float mma_products_above(const das_problem &pb) {
+    const float places = (float)((pb.S + 3) / 4 * 4) / (float)pb.S;
+    return 100.f / ((float)pb.B * places);
+}
+
 // 4-D map over x: samples, events, channels, items; box {64, 1, 1, items},
 // 128-byte swizzle; samples and items past the end read as zeros.
 static ffdas_error_t sample_map(CUtensorMap &map, const void *x, const das_problem &pb, int64_t bs, int64_t cs, int64_t ss,
@@ -33,7 +47,8 @@ static ffdas_error_t sample_map(CUtensorMap &map, const void *x, const das_probl
     return r == CUDA_SUCCESS ? FFDAS_SUCCESS : FFDAS_ERROR_CUDA_DRIVER;
 }
 
-ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call &a, float *out) {
+ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call &a, float *out, void *made,
+                         const int *run_if) {
     // items per CTA: at most 256 columns of tensor memory per product, evenly
     const int groups = (pb.B + 255) / 256;
     const int items = ((pb.B + groups - 1) / groups + 15) / 16 * 16;
@@ -49,13 +64,13 @@ ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call
     const size_t packed = aligned ? 0 : (size_t)pb.B * pb.C * pb.S * npad * sizeof(__half);
     workspace W(h);
     FFDAS_TRY(W.alloc(packed + 512));
-    char *plan = W.get<char>() + ((packed + 255) & ~size_t(255));
+    void *plan = W.get<char>() + ((packed + 255) & ~size_t(255));
     if (!aligned) {
         __half *xp = W.get<__half>();
         const dim3 grid((unsigned)((npad / 8 + 255) / 256), (unsigned)std::min(pb.S, 65535),
                         (unsigned)std::min<int64_t>((int64_t)pb.B * pb.C, 65535));
         mma_repack_kernel<<<grid, 256, 0, h.stream>>>(x, pb.x_bstride, pb.x_cstride, pb.x_sstride, pb.C, pb.S, pb.N,
-                                                      pb.B * pb.C, (int)npad, xp);
+                                                      pb.B * pb.C, (int)npad, xp, run_if);
         FFDAS_TRY(ffdas_launch_check(h.stream));
         x = xp;
         ss = npad;
@@ -63,11 +78,14 @@ ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call
         bs = npad * pb.S * pb.C;
     }
 
-    FFDAS_TRY(launch_tile_plan(h, make_plan(pb, ST_F16, a.srcpos, a.dstpos, a.offsets, pb.N, kMmaTile, kPlanMma, plan)));
+    if (!made)
+        FFDAS_TRY(launch_tile_plan(h, make_plan(pb, ST_F16, a.srcpos, a.dstpos, a.offsets, pb.N, kMmaTile, kPlanMma, plan)));
 
     mma_params p;
     std::memset(&p, 0, sizeof(p));
-    p.plan = reinterpret_cast<const tile_plan *>(plan);
+    p.plan = static_cast<const tile_plan *>(made ? made : plan);
+    p.nonfinite = &static_cast<tile_plan *>(made ? made : plan)->nonfinite;
+    p.run_if = run_if;
     p.srcpos = a.srcpos; p.dstpos = a.dstpos; p.offsets = a.offsets; p.weights = a.weights;
     p.srcdir = reinterpret_cast<const float4 *>(a.srcdir);
     p.C = pb.C; p.S = pb.S; p.N = pb.N; p.B = pb.B; p.items = items; p.V = pb.V;
@@ -87,8 +105,6 @@ ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call
     if (z <= 1) p.cchunk = 0;
     else if (pb.out_bstride == pb.V) FFDAS_CUDA(cudaMemsetAsync(out, 0, (size_t)pb.B * pb.V * sizeof(float), h.stream));
     else FFDAS_TRY(launch_scale_image(h, pb, out, 0.f, 1));
-    p.nonfinite = reinterpret_cast<int *>(plan + 64);
-    FFDAS_CUDA(cudaMemsetAsync(p.nonfinite, 0, sizeof(int), h.stream));
 
     CUtensorMap map;
     std::memset(&map, 0, sizeof(map));

@@ -52,12 +52,13 @@
 #include <cuda_fp16.h>
 
 #include "das_common.cuh"
+#include "das_problem.h"
 #include "das_staged.cuh"
 #include "gram_tc.cuh"
 
 namespace ffdas {
 
-constexpr int kMmaTile = 256;      // voxels per CTA
+constexpr int kMmaTile = kMmaTileVoxels;   // voxels per CTA
 constexpr int kMmaW = 64;          // samples per window: one 128-byte row
 constexpr int kMmaStep = 56;       // taps of a window: first samples k0 .. k0 + 55
 constexpr int kMmaBuilders = 256;  // threads that build one buffer
@@ -80,6 +81,7 @@ struct mma_params {
     int64_t out_bstride;
     int *status;
     int *nonfinite;                 // set when a value added to the image is not finite
+    const int *run_if;              // device word without which nothing is done, or null
 };
 
 constexpr size_t mma_smem_bytes(int items) {
@@ -137,6 +139,7 @@ __device__ __forceinline__ int mma_count(int len) { return len > 1 ? (len - 1 + 
 __global__ void __launch_bounds__(kMmaThreads, 1) das_mma_kernel(const __grid_constant__ CUtensorMap map,
                                                                  const mma_params params) {
     mma_params p = params;
+    if (p.run_if && *p.run_if == 0) return;   // uniform over the grid
     if (p.plan) {
         p.T0 = p.plan->T0; p.T1 = p.plan->T1; p.n0 = p.plan->n0; p.n1 = p.plan->n1;
         if ((int64_t)blockIdx.x >= (int64_t)p.n0 * p.n1 * p.D2) return;
@@ -479,9 +482,9 @@ __global__ void __launch_bounds__(256) mma_fixup_kernel(const mma_params p, cons
 // rows TMA cannot read in place.
 __global__ void __launch_bounds__(256) mma_repack_kernel(const __half *__restrict__ x, int64_t bstride, int64_t cstride,
                                                          int64_t sstride, int C, int S, int N, int BC, int Npad,
-                                                         __half *__restrict__ out) {
+                                                         __half *__restrict__ out, const int *run_if) {
     const int k0 = (blockIdx.x * 256 + threadIdx.x) * 8;
-    if (k0 >= Npad) return;
+    if (k0 >= Npad || (run_if && *run_if == 0)) return;
     for (int s = blockIdx.y; s < S; s += gridDim.y)
         for (int bc = blockIdx.z; bc < BC; bc += gridDim.z) {
             const __half *r = x + (int64_t)(bc / C) * bstride + (int64_t)(bc % C) * cstride + (int64_t)s * sstride;

@@ -201,10 +201,12 @@ template <typename Tin, int K>
 __global__ void __launch_bounds__(kIngestThreads) ingest_pairs_kernel(
     const Tin *__restrict__ x, int64_t bstride, int64_t cstride, int64_t sstride,
     int C, int S, int N, int BC, int64_t Npad,
-    typename pair_traits<K>::storage *__restrict__ P, const float *__restrict__ gain, int gain_bstride) {
+    typename pair_traits<K>::storage *__restrict__ P, const float *__restrict__ gain, int gain_bstride,
+    const int *skip) {
     using st = typename pair_traits<K>::storage;
     using W = typename sample_io<Tin>::w;
     static_assert(sizeof(pair_quad<st>) == kIngestVec * sizeof(st), "pair_quad packing");
+    if (skip && *skip) return;   // no kernel reads the pairs (not launched beside the plan then)
     const int64_t k0 = ((int64_t)blockIdx.x * kIngestThreads + threadIdx.x) * kIngestVec;
     if (k0 >= Npad) return;   // Npad is a multiple of kIngestVec
     for (int s = blockIdx.y; s < S; s += gridDim.y) {

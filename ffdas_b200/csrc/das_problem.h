@@ -132,7 +132,14 @@ ffdas_error_t launch_staged_bwd(ffdas_context &h, const das_problem &pb, int kin
 // Large half-precision batches on the tensor cores (csrc/das_mma.cuh), straight
 // from x: half data at its default precision, FP32 output, beta 0.
 bool mma_supported(const das_problem &pb, ffdas_datatype_t xt, ffdas_datatype_t ot, int kind);
-ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call &a, float *out);
+// Relative time of the batch tiles (plan_params::products_above) from which the
+// products are faster; below 1 they are faster in any case.
+float mma_products_above(const das_problem &pb);
+constexpr int kMmaTileVoxels = 256;
+// plan, run_if: a plan made by the caller, and a device word without which the
+// products do nothing.
+ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call &a, float *out, void *plan = nullptr,
+                         const int *run_if = nullptr);
 
 // das_sparse on sorted list entries (csrc/das_entries.cuh): real storage kinds,
 // f32 output, lists of at most 64 entries over at most 480 events; no pair

@@ -269,8 +269,10 @@ ffdas_error_t launch_staged(ffdas_context &h, const das_problem &pb, int kind, c
     if (gp.cchunk) {   // channel slices add into the image: prepare it (beta * out, or 0)
         if (grid.z < 2) return FFDAS_ERROR_INTERNAL;
         dim3 sg((unsigned)((pb.V + 255) / 256), (unsigned)std::min(pb.B, 65535));
+        // (not where the plan left the image to the tensor-core products)
+        const int *off = gp.plan ? &static_cast<const tile_plan *>(gp.plan)->products : nullptr;
         scale_image_kernel<<<sg, 256, 0, h.stream>>>(static_cast<float *>(gp.out), pb.out_bstride, pb.V, pb.B,
-                                                     (float)gp.beta_re, gp.beta_zero, nullptr);
+                                                     (float)gp.beta_re, gp.beta_zero, off);
         FFDAS_TRY(ffdas_launch_check(h.stream));
     }
     // (the 256-voxel kernel of one item reads no plan: it would run for both widths)

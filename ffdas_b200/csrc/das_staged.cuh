@@ -50,7 +50,9 @@ constexpr int kStatusTimeout = 1;
 // kernels run.  One instance per window width is launched; the other exits.
 struct __align__(16) tile_plan {
     int T0, T1, n0, n1;   // T2 = 1
-    int wb;
+    int wb;               // 0: no staged instance runs, the tensor-core products do
+    int products;         // 1 then
+    int nonfinite;        // 0 here; set by the products where a value is not finite
 };
 
 struct staged_params {

@@ -33,6 +33,9 @@ constexpr float kPlanSlow = 1.7f, kPlanSlowAdjoint = 4.f;
 // per SM (784 channels, 3 waves, 96 x 86 x 86 voxels: 1.21 to 1.34 ms); in the
 // adjoints the gradient bins double as well
 constexpr float kPlanWide = 1.15f, kPlanWideAdjoint = 1.3f;
+// Batch tiles whose windows all overflow against ones whose windows fit: 5.4 times
+// the time (56 items, 192 channels, 8 events, 100 x 64 pixels: 2.78 ms).
+constexpr float kPlanSlowBatch = 4.4f;
 
 struct plan_params {
     const float *srcpos, *dstpos, *offsets;
@@ -42,6 +45,7 @@ struct plan_params {
     int shapes;
     int T0[kPlanShapes], T1[kPlanShapes];
     int mode;   // kPlanForward, kPlanBatch, kPlanAdjoint or kPlanMma
+    float products_above;   // kPlanBatch: padding x overflow above which the products run (0: never)
     tile_plan *plan;
 };
 
@@ -113,13 +117,14 @@ __device__ __forceinline__ void tile_plan_block(const plan_params &q) {
     // a lane per (shape, width); the least cost wins, ties to the lower lane
     constexpr float kSamples = (float)(kPlanAnchors * kPlanEvents * kPlanChannels);
     const int i = tid >> 1, wb = (tid & 1) ? 64 : 32;
-    float cost = INFINITY;
+    float cost = INFINITY, batch = 0.f;
     if (i < q.shapes) {
         const int n0 = (q.D0 + q.T0[i] - 1) / q.T0[i], n1 = (q.D1 + q.T1[i] - 1) / q.T1[i];
         const float waste = (float)(n0 * q.T0[i]) * (float)(n1 * q.T1[i]) / ((float)q.D0 * (float)q.D1);
         int n = 0;
         for (int a = 0; a < kPlanAnchors; a++) n += __popc(over[tid & 1][i][a]);
         const float slow = (float)n / (float)(kPlanAnchors * kPlanChannels);
+        batch = waste * (1.f + kPlanSlowBatch * slow);
         if (q.mode == kPlanMma) {
             // the products grow with the windows, whatever their width; the
             // image is read and written in rows of T0 voxels
@@ -150,6 +155,7 @@ __device__ __forceinline__ void tile_plan_block(const plan_params &q) {
             best = l;
         }
     }
+    batch = __shfl_sync(0xffffffffu, batch, best);
     if (tid != 0) return;
     const int k = best >> 1;
     tile_plan pl;
@@ -157,7 +163,9 @@ __device__ __forceinline__ void tile_plan_block(const plan_params &q) {
     pl.T1 = q.T1[k];
     pl.n0 = (q.D0 + pl.T0 - 1) / pl.T0;
     pl.n1 = (q.D1 + pl.T1 - 1) / pl.T1;
-    pl.wb = (best & 1) ? 64 : 32;
+    pl.products = q.products_above > 0.f && batch > q.products_above;
+    pl.wb = pl.products ? 0 : ((best & 1) ? 64 : 32);
+    pl.nonfinite = 0;
     *q.plan = pl;
 }
 

@@ -176,7 +176,8 @@ typedef struct {
 /* What the last das/das_sparse/backward call on a handle launched (new).
  * variant of a forward: 1 gather, 2 TMA-staged (real data, or complex data on
  * batch tiles), 5 direct, 6 das_sparse over bucketed lists, 9 das_sparse over
- * sorted entries, 10 half-precision batches on the tensor cores; of an adjoint:
+ * sorted entries, 10 half-precision batches on the tensor cores (or, where the
+ * plan made on the device finds them faster, on batch tiles); of an adjoint:
  * see ffdas_das_backward.  A call without a schedule chooses the tile shape
  * and window width of the staged kernels on the device: tile_x then holds the
  * voxels of a tile (tile_y = tile_z = 1), event_chunk that of the 32-sample

@@ -153,7 +153,7 @@ def _with_config(config, f, *args, **kw):
 
 
 @pytest.mark.parametrize("dtype,B,S,C", [(torch.float32, 1, 5, 1200), (torch.float32, 3, 4, 200), (torch.complex64, 1, 4, 33),
-                                         (torch.complex64, 3, 5, 20), (torch.float16, 32, 3, 33)], ids=str)
+                                         (torch.complex64, 3, 5, 20), (torch.float16, 96, 3, 33)], ids=str)
 @pytest.mark.parametrize("far", [2.0 ** 22, 2.0 ** 28])
 def test_far_delays_that_cancel_far_distances(dtype, B, S, C, far):
     # distances round to 0.5 and to 32 samples: every kernel takes the same taps as
@@ -360,7 +360,8 @@ def test_tensor_core_batches_many_drains(V, C, S, late):
     # up to 780 (channel, event) pairs per CTA, with (1240 voxels) and without (37888: a tile an SM)
     # channel slices; `late`: the last channels lie outside the record, and no window
     # follows the last drain
-    x, src, dst, offs, w = _problem(32, C, S, 256, *V, (0.5, 0.5), dtype=torch.float16, seed=late)
+    B = 32 if S == 1 else 96   # (fewer items of three events may take the batch tiles)
+    x, src, dst, offs, w = _problem(B, C, S, 256, *V, (0.5, 0.5), dtype=torch.float16, seed=late)
     if late:
         src[C - late:, 2] = 1e6
     args = _dev(x, src, dst, offs, w)
@@ -386,12 +387,31 @@ def test_tensor_core_batches_many_drains(V, C, S, late):
 def test_tensor_core_batches_are_no_less_exact_than_the_pair_kernels(C, S, N):
     # 22-bit weights and truncated sums against FP32 weights and sums, on the same
     # data, both against the oracle
-    x, src, dst, offs, w = _problem(32, C, S, N, 37, 59, (0.2 * N / 37, 0.5), dtype=torch.float16, seed=C)
+    x, src, dst, offs, w = _problem(96, C, S, N, 37, 59, (0.2 * N / 37, 0.5), dtype=torch.float16, seed=C)
     args, ref = _dev(x, src, dst, offs, w), _oracle(x, src, dst, offs, w)
     got = ffdas_b200.das(*args)
     assert _info()["variant"] == 10
     pairs = _with_config({"variant": 1}, ffdas_b200.das, *args)
     assert oracle.rel_l2(got.cpu().numpy(), ref) <= oracle.rel_l2(pairs.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("B,C,S,N,pitch", [(32, 40, 4, 256, (0.4, 0.5)), (33, 40, 4, 250, (12.0, 9.0)), (40, 150, 3, 504, (0.5, 0.4)),
+                                           (40, 150, 3, 501, (15.0, 15.0)), (64, 20, 5, 256, (3.0, 2.0))], ids=str)
+def test_batches_on_the_products_or_the_batch_tiles(B, C, S, N, pitch):
+    # few items: fine pitches leave the image to the batch tiles, coarse ones, whose
+    # windows overflow, to the products; both launched, with channel slices and without
+    x, src, dst, offs, w = _problem(B, C, S, N, 131, 67, pitch, dtype=torch.float16, seed=B + S)
+    args = _dev(x, src, dst, offs, w)
+    out = torch.full((B, 131, 67), float("nan"), device=DEV)
+    for srcdir in (None, _cone(C).to(DEV)):
+        ffdas_b200.das(*args, srcdir=srcdir, out=out)
+        assert _info()["variant"] == 10
+        ref = _with_config({"variant": 1}, ffdas_b200.das, *args, srcdir=srcdir)
+        # (each is off 64 bits by less than TOL)
+        assert oracle.rel_l2(out.cpu().numpy(), ref.cpu().numpy()) < 2 * TOL
+        few = _oracle(x, src, dst[::13, ::7].contiguous(), offs[:, ::13, ::7].contiguous(), w[:, ::13, ::7].contiguous(),
+                      srcdir=None if srcdir is None else _cone(C))
+        assert oracle.rel_l2(out[:, ::13, ::7].cpu().numpy(), few) < TOL
 
 
 def test_tensor_core_batches_channels_trailing_view_and_non_finite_values():
@@ -430,7 +450,8 @@ def test_pair_buffer_only_where_the_backward_reads_it(kind, variant, kept):
     assert torch.isfinite(offs.grad).all() and offs.grad.abs().max() > 0
 
 
-_CAPTURED = dict(staged=(1, 1200, 4, torch.float32, 2), batch=(3, 200, 3, torch.float32, 2), products=(33, 40, 3, torch.float16, 10),
+_CAPTURED = dict(staged=(1, 1200, 4, torch.float32, 2), batch=(3, 200, 3, torch.float32, 2), products=(96, 12, 3, torch.float16, 10),
+                 either=(33, 40, 3, torch.float16, 10),
                  iq=(3, 20, 4, torch.complex64, 2), iq_copied=(1, 20, 1, torch.complex64, 2), entries=(4, 1000, 4, torch.float32, 9))
 
 
