@@ -585,12 +585,6 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
                              asked ? h.config.tile_x : 0);
     }
 
-    // ---- large half-precision batches: tensor cores, straight from x; where the
-    // batch tiles can be faster (products_above) both are launched below and the
-    // plan of the batch tiles decides which of them runs ----
-    const bool contested = way == route::mma && mma_products_above(pb) >= 1.f;
-    if (way == route::mma && !contested) return launch_mma(h, pb, a, static_cast<float *>(a.out));
-
     // ---- dense complex (IQ) data without a schedule: batch tiles on windows of
     // plain samples (das_iq.cuh).  (A pair buffer stays unfilled: the adjoint of
     // such a call reads no pairs.)
@@ -642,6 +636,24 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
         return err;
     }
 
+    // without a schedule the staged kernels' tile shape and window width follow
+    // the geometry (das_tile_plan.cuh): batch tiles and the 512-voxel tiles of one
+    // item read a plan; the 256-voxel kernel of a batch that cannot have TMA boxes
+    // does not
+    const bool staged_ok = staged_supported(pb, kind) && od.dtype == FFDAS_R_32F;
+    const schedule s = plan_schedule(h, pb, kind, staged_ok);
+    const int tile_voxels = s.T0 * s.T1 * s.T2;
+    const bool reads_plan = s.variant == 2 && !h.has_config && (s.BT > 1 || tile_voxels == 512);
+    const int plan_tile = reads_plan ? tile_voxels : 0;
+    const int64_t plan_tiles = plan_tile && pb.C > 0 ? plan_max_tiles(pb, plan_tile) : 0;
+    const bool planned = plan_tiles > 0 && plan_tiles <= INT32_MAX;
+
+    // ---- large half-precision batches: tensor cores, straight from x; where the
+    // batch tiles can be faster (products_above) both are launched below and the
+    // plan of the batch tiles decides which of them runs ----
+    const bool contested = way == route::mma && planned && s.BT > 1 && mma_products_above(pb) >= 1.f;
+    if (way == route::mma && !contested) return launch_mma(h, pb, a, static_cast<float *>(a.out));
+
     // ---- ingest: x -> pair rows (workspace) ----
     const int64_t npad = pair_row_length(pb.N);
     const int64_t rows = (int64_t)pb.B * pb.C * pb.S;
@@ -652,25 +664,13 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     void *Pbase = nullptr;
     if (h.pair_buf && h.pair_buf_bytes >= pair_bytes + 256) {
         Pbase = h.pair_buf;
-    } else if (contested && P.alloc(pair_bytes + 256) != FFDAS_SUCCESS) {
-        return launch_mma(h, pb, a, static_cast<float *>(a.out));   // no room for pairs: none needed
-    } else if (contested) {
-        Pbase = P.get<void>();
     } else {
-        FFDAS_TRY(P.alloc(pair_bytes + 256));   // after the pairs: das_sparse's gate word, the tile plan
+        const ffdas_error_t e = P.alloc(pair_bytes + 256);   // after the pairs: das_sparse's gate word, the tile plans
+        if (e != FFDAS_SUCCESS && contested) return launch_mma(h, pb, a, static_cast<float *>(a.out));   // needs no pairs
+        FFDAS_TRY(e);
         Pbase = P.get<void>();
     }
-    // without a schedule the staged kernels' tile shape and window width follow
-    // the geometry (das_tile_plan.cuh)
-    const bool staged_ok = staged_supported(pb, kind) && od.dtype == FFDAS_R_32F;
-    const schedule s = plan_schedule(h, pb, kind, staged_ok);
-    // (batch tiles and the 512-voxel tiles of one item read a plan; the 256-voxel
-    // kernel of a batch that cannot have TMA boxes does not)
-    const bool planned = s.variant == 2 && !h.has_config && (s.BT > 1 || s.T0 * s.T1 * s.T2 == 512);
-    const int plan_tile = planned ? s.T0 * s.T1 * s.T2 : 0;
-    const int64_t plan_tiles = plan_tile && pb.C > 0 ? plan_max_tiles(pb, plan_tile) : 0;
-    void *const plan = plan_tiles > 0 && plan_tiles <= INT32_MAX ? static_cast<char *>(Pbase) + pair_bytes + 64 : nullptr;
-    if (contested && (!plan || s.BT == 1)) return launch_mma(h, pb, a, static_cast<float *>(a.out));
+    void *const plan = planned ? static_cast<char *>(Pbase) + pair_bytes + 64 : nullptr;
     const int *products = nullptr;   // device word: the products run, not the batch tiles
     if (plan) {
         plan_params own = make_plan(pb, kind, a.srcpos, a.dstpos, a.offsets, npad, plan_tile,

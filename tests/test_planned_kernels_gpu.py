@@ -412,6 +412,14 @@ def test_batches_on_the_products_or_the_batch_tiles(B, C, S, N, pitch):
         few = _oracle(x, src, dst[::13, ::7].contiguous(), offs[:, ::13, ::7].contiguous(), w[:, ::13, ::7].contiguous(),
                       srcdir=None if srcdir is None else _cone(C))
         assert oracle.rel_l2(out[:, ::13, ::7].cpu().numpy(), few) < TOL
+    if B == 64:   # (on the products in any case)
+        return
+    _lib.load().ffdas_debug_fail_alloc_after(1)   # no room for pair rows: the products need none
+    try:
+        got = ffdas_b200.das(*args, srcdir=srcdir)
+    finally:
+        _lib.load().ffdas_debug_fail_alloc_after(0)
+    assert _info()["kernels"] <= 5 and oracle.rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < 2 * TOL
 
 
 def test_tensor_core_batches_channels_trailing_view_and_non_finite_values():
