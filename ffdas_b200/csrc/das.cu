@@ -651,7 +651,7 @@ ffdas_error_t das_forward(ffdas_context &h, const das_call &a) {
     // ---- large half-precision batches: tensor cores, straight from x; where the
     // batch tiles can be faster (products_above) both are launched below and the
     // plan of the batch tiles decides which of them runs ----
-    const bool contested = way == route::mma && planned && s.BT > 1 && mma_products_above(pb) >= 1.f;
+    const bool contested = way == route::mma && planned && s.BT > 1 && mma_products_above(pb) > 0.f;
     if (way == route::mma && !contested) return launch_mma(h, pb, a, static_cast<float *>(a.out));
 
     // ---- ingest: x -> pair rows (workspace) ----

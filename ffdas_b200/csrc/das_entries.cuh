@@ -30,7 +30,7 @@
 // (delays change by at most one sample per wavelength of distance, which bounds
 // the transmit part).
 //
-// Measured on that frame: sort 37 us, this kernel 357 us, against 656 us for the
+// Measured on that frame: sort 38 us, this kernel 351 us, against 656 us for the
 // gather kernel and 32 for its ingest.  Below 2^27 list places x channels x items
 // (2^24 from 256 channels on) the gather kernel's shorter chain wins (138 channels,
 // 12 of 24 events, 166 x 170 pixels: 109 against 149 us), and with under a quarter of the events listed a window serves too few

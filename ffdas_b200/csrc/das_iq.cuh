@@ -23,7 +23,7 @@
 // L2 and shared memory, and an ingest of x (40 us of 343 for 4 frames of 128
 // channels, 8 plane waves, 2048 samples), for one subtraction a tap less.
 //
-// Measured on those frames, 256 x 256 pixels: 215 us, where the gather kernel
+// Measured on those frames, 256 x 256 pixels: 207 us, where the gather kernel
 // with a sine and cosine per tap took 538 us and its ingest 40; the adjoint of
 // two frames, 192 x 256 pixels, 358 us against 1886 for the gather form with
 // global atomics.

@@ -26,11 +26,13 @@ bool mma_supported(const das_problem &pb, ffdas_datatype_t xt, ffdas_datatype_t 
 // 150 x 200, 64: 685 and 672; 192, 9, 299 x 102, 81: 2726 and 2572; 64, 3, 400 x 256,
 // 81: 661 and 809; 128, 8, 200 x 100, 128: 993 and 1265), and windows that overflow cost
 // the batch tiles up to 5.4 times that (192, 8, 100 x 64, 56: 953 and 2780).  Both are
-// launched below 100: what the loser costs, 12 us on a call of 300 and 20 on one of 100,
-// buys the choice.
+// launched below 100 (what the loser costs, 12 us on a call of 300 and 20 on one of 100,
+// buys the choice), and the products run from a padding and overflow on that bring the
+// items to 112 (48 items, 192, 2, 299 x 102: 625 and 537).
 float mma_products_above(const das_problem &pb) {
     const float places = (float)((pb.S + 3) / 4 * 4) / (float)pb.S;
-    return 100.f / ((float)pb.B * places);
+    const float items = (float)pb.B * places;
+    return items < 100.f ? 112.f / items : 0.f;
 }
 
 // 4-D map over x: samples, events, channels, items; box {64, 1, 1, items},
@@ -67,8 +69,10 @@ ffdas_error_t launch_mma(ffdas_context &h, const das_problem &pb, const das_call
     void *plan = W.get<char>() + ((packed + 255) & ~size_t(255));
     if (!aligned) {
         __half *xp = W.get<__half>();
-        const dim3 grid((unsigned)((npad / 8 + 255) / 256), (unsigned)std::min(pb.S, 65535),
-                        (unsigned)std::min<int64_t>((int64_t)pb.B * pb.C, 65535));
+        dim3 grid((unsigned)((npad / 8 + 255) / 256), (unsigned)std::min(pb.S, 65535),
+                  (unsigned)std::min<int64_t>((int64_t)pb.B * pb.C, 65535));
+        // blocks that may have nothing to do are few, and walk the rows
+        if (run_if) grid.z = std::min(grid.z, std::max(1u, 4096u / (grid.x * grid.y)));
         mma_repack_kernel<<<grid, 256, 0, h.stream>>>(x, pb.x_bstride, pb.x_cstride, pb.x_sstride, pb.C, pb.S, pb.N,
                                                       pb.B * pb.C, (int)npad, xp, run_if);
         FFDAS_TRY(ffdas_launch_check(h.stream));

@@ -133,7 +133,7 @@ ffdas_error_t launch_staged_bwd(ffdas_context &h, const das_problem &pb, int kin
 // from x: half data at its default precision, FP32 output, beta 0.
 bool mma_supported(const das_problem &pb, ffdas_datatype_t xt, ffdas_datatype_t ot, int kind);
 // Relative time of the batch tiles (plan_params::products_above) from which the
-// products are faster; below 1 they are faster in any case.
+// products are faster; 0: they are, or may be, in any case.
 float mma_products_above(const das_problem &pb);
 constexpr int kMmaTileVoxels = 256;
 // plan, run_if: a plan made by the caller, and a device word without which the
